@@ -89,6 +89,7 @@ struct fss_ctx {
     std::vector<double> leaf_theta;
     int nmax = 0, level_mask = 0;
     int parts = 1;
+    double list_blocks = 1, list_sources = 0;  // pair blocks over all leaves, the sources each goes through
     int64_t pstride = 0;  // partial slot stride: n, or n + proxy slots with target clusters
     int n_up_blocks = 0, n_dn_blocks = 0;  // blocks of the batched V^-1 products
     int down_max_deg = 0;                  // highest target-cluster degree

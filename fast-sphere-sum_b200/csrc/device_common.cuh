@@ -91,12 +91,18 @@ __device__ __forceinline__ float lg2_fast(float x) {
     return y;
 }
 
+// The hardware's approximation of an FP64 reciprocal (about 20 bits).
+__device__ __forceinline__ double rcp_seed(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+
 // FP64 reciprocal: hardware approximation refined by two Newton-Raphson
 // steps y <- y + y (1 - x y) (quadratic convergence from the approximation's
 // ~2^-20 relative error to below FP64 rounding).
 __device__ __forceinline__ double rcp_fast(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double y = rcp_seed(x);
     double e = fma(-x, y, 1.0);
     y = fma(y, e, y);
     e = fma(-x, y, 1.0);

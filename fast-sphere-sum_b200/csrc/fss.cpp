@@ -149,11 +149,32 @@ int src_size_ensure(fss_ctx* c, int64_t count) {
     return FSS_OK;
 }
 
+// FP64 engine: the number of parts of a source list, for `blocks` blocks that
+// go through `sources` sources each, that takes the least time where an SM
+// shares its FP64 pipe between its blocks and up to three run side by side
+// unhindered, and a block's start and final sum cost as much as 100 sources.
+// Measured against every split of 1 to 16 (us per right-hand side, FP64
+// treecode): 20 leaves of 128 16 parts 62.1 (4 parts 65.1), 80 leaves of 250
+// 12 parts 167.9 (4: 205.3), 320 of 128 5 parts 242 (4: 243.7), 1280 of 128 3
+// parts 981 (2: 1003.5); never more than 2% behind the best one.
+int plane_parts(double blocks, double sources, int most) {
+    int best = 1;
+    double best_t = 1e300;
+    for (int p = 1; p <= most; p++) {
+        const double t = std::max(3.0, std::ceil(blocks * p / 148.0)) * (sources / p + 100.0);
+        if (t < best_t) {
+            best_t = t;
+            best = p;
+        }
+    }
+    return best;
+}
+
 // Lists of the direct sum: blocks of targets x P chunks of the sources.
 int build_direct_lists(fss_ctx* c) {
     const int64_t n = c->n;
     c->shape = pairs_shape(c->fp64, c->cfg.block_threads, c->cfg.targets_per_thread);
-    const int TB = c->shape.targets();
+    const int TB = c->fp64 ? kChunkTargets : c->shape.threads - 32;
     const int64_t tiles = (n + TB - 1) / TB;
     int P = c->cfg.src_parts;
     if (P <= 0) {
@@ -161,6 +182,7 @@ int build_direct_lists(fss_ctx* c) {
         P = int(std::max<int64_t>(1, (want + tiles - 1) / std::max<int64_t>(tiles, 1)));
         P = int(std::min<int64_t>(P, std::max<int64_t>(1, n / 512)));
         P = std::min(P, 64);
+        if (c->fp64) P = plane_parts(double(tiles), double(n), int(std::min<int64_t>(64, std::max<int64_t>(1, n / 64))));
     }
     c->parts = P;
     ListOutput& L = c->lists;
@@ -194,6 +216,28 @@ int build_direct_lists(fss_ctx* c) {
     TRY(src_size_ensure(c, n));
     c->pstride = n;
     CU(c->partials.ensure(sizeof(double4) * size_t(P) * size_t(std::max<int64_t>(n, 1))));
+    if (c->fp64) {  // order_sources
+        CU(c->key.ensure(sizeof(uint32_t) * n));
+        CU(c->key_tmp.ensure(sizeof(uint32_t) * n));
+        CU(c->sortq.ensure(sizeof(int32_t) * n));
+        CU(c->vals_tmp.ensure(sizeof(int32_t) * n));
+        CU(c->hist.ensure(sizeof(uint32_t) * sort_scratch_words(n)));
+    }
+    return FSS_OK;
+}
+
+// FP64 direct sum: the spatial order of the stage state and its sources in
+// it, at the start of every evaluation of new positions (an RK4 step, a
+// right-hand side): the order, and so every result, depends on the positions
+// alone.
+bool ordered(const fss_ctx* c) { return !c->tree && c->fp64; }
+int order_sources(fss_ctx* c) {
+    if (!ordered(c)) return FSS_OK;
+    ProfScope ps(c, "order", order_launch_count(c->n));
+    launch_order(c->stream, c->n, c->xs.as<double4>(), c->area_s.as<double>(), c->key.as<uint32_t>(),
+                 c->key_tmp.as<uint32_t>(), c->sortq.as<int32_t>(), c->vals_tmp.as<int32_t>(), c->hist.as<uint32_t>(),
+                 c->src.as<double4>());
+    CU(cudaGetLastError());
     return FSS_OK;
 }
 
@@ -237,6 +281,24 @@ void make_lists(fss_ctx* c) {
     }
 }
 
+// What the FP64 source split is chosen by: blocks (leaves that hold
+// particles) and the mean count of sources they go through, over all leaves
+// (also those that other ranks own).
+void list_size(fss_ctx* c) {
+    double blocks = 0, sources = 0;
+    for (int64_t lf = 0; lf < c->nleaf; lf++) {
+        const int k = chunk_count(c->leaf_start_h[lf + 1] - c->leaf_start_h[lf]);
+        if (k == 0) continue;
+        double n = 0;
+        for (const ASrc& a : c->alists[lf])
+            n += a.proxy ? double(nproxy(a.deg)) : double(c->counts_h[c->geom.lev_off[a.level] + a.node]);
+        blocks += 1;
+        sources += k * n;
+    }
+    c->list_blocks = std::max(blocks, 1.0);
+    c->list_sources = sources / c->list_blocks;
+}
+
 // Sharded treecode: the units are the faces of the shallowest level holding
 // a target cluster (every target cluster and the downward pass below it then
 // lie within one unit), or the leaves; each unit costs the interactions of
@@ -245,6 +307,7 @@ void make_lists(fss_ctx* c) {
 // plan from the same tree), and this rank keeps the source lists of its own
 // leaves and clusters only.
 int shard_filter(fss_ctx* c) {
+    list_size(c);
     if (c->shard_nranks <= 0) return FSS_OK;
     const int LL = c->leaf_level;
     int u = LL;
@@ -448,11 +511,12 @@ int build_tree(fss_ctx* c) {
     return FSS_OK;
 }
 
-// Block shape for the treecode's pair kernel: the configured one, or the
-// smallest supported block whose consumer threads cover the largest leaf (so
-// that no leaf needs a second chunk).
+// Block shape for the treecode's pair kernel: the configured one, or (FP32)
+// the smallest supported block whose consumer threads cover the largest leaf
+// (so that no leaf needs a second chunk).
 PairShape choose_shape(fss_ctx* c) {
     if (c->cfg.block_threads > 0) return pairs_shape(c->fp64, c->cfg.block_threads, c->cfg.targets_per_thread);
+    if (c->fp64) return pair_shapes(true).front();
     int maxleaf = 1;
     for (int64_t l = 0; l < c->nleaf; l++) maxleaf = std::max(maxleaf, c->leaf_start_h[l + 1] - c->leaf_start_h[l]);
     for (const PairShape& sh : pair_shapes(c->fp64))
@@ -472,15 +536,19 @@ int materialize(fss_ctx* c, PairShape shape) {
     in.n = n;
     in.leaf_start = c->leaf_start_h.data();
     in.tile = shape.tile;
-    in.threads = shape.targets();
-    in.per_thread = 1;
     int P = c->cfg.src_parts;
     if (P <= 0) {
+        // blocks of targets: the smallest of these that holds the largest leaf
+        int maxleaf = 1, TB = 256;
+        for (int64_t l = 0; l < c->nleaf; l++) maxleaf = std::max(maxleaf, c->leaf_start_h[l + 1] - c->leaf_start_h[l]);
+        for (int tb : {192, 160, 128})
+            if (tb >= maxleaf) TB = tb;
+        if (c->cfg.block_threads > 0) TB = shape.threads - 32;
         int64_t chunks = 0;
-        const int TB = in.threads * in.per_thread;
         for (int64_t l = 0; l < c->nleaf; l++) chunks += (c->leaf_start_h[l + 1] - c->leaf_start_h[l] + TB - 1) / TB;
         const double waves = double(chunks) / (148.0 * 8.0);
         P = waves >= 3.0 ? 1 : (waves >= 1.0 ? 2 : 4);
+        if (c->fp64) P = plane_parts(c->list_blocks, c->list_sources, 16);
     }
     in.parts = P;
     in.all_leaves = c->resort;
@@ -686,6 +754,7 @@ int eval(fss_ctx* c, EpiArgs& ea, bool want_psi) {
     ea.area = c->area_s.as<double>();
     ea.wtotal = c->wtotal.as<double>();
     ea.perm = c->tree ? c->perm.as<int32_t>() : nullptr;
+    ea.order = ordered(c) ? c->sortq.as<int32_t>() : nullptr;
     ea.src = c->src.p;
     ea.leaf_of = nullptr;
     ea.frame = nullptr;  // interaction sources in absolute coordinates
@@ -849,6 +918,7 @@ int resort(fss_ctx* c) {
 
 int rk4_once(fss_ctx* c, double dt, double omega) {
     if (c->tree && c->resort) TRY(resort(c));
+    TRY(order_sources(c));
     for (int stage = 1; stage <= 4; stage++) {
         EpiArgs ea;
         ea.mode = EPI_RK4;
@@ -905,6 +975,7 @@ int rhs_host(fss_ctx* c, const double* state5, const double* area, double omega,
     CU(cudaMemcpyAsync(c->in5.p, state5, sizeof(double) * 5 * c->n, cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemcpyAsync(c->area_in.p, area, sizeof(double) * c->n, cudaMemcpyHostToDevice, c->stream));
     TRY(gather(c, false));
+    TRY(order_sources(c));
     c->stage_dirty = true;
     EpiArgs ea;
     ea.mode = EPI_RHS;
@@ -957,6 +1028,7 @@ int internal_relist(fss_ctx* c) {
 // Velocity of the current stage state into a host array (caller's order).
 int internal_rhs_current(fss_ctx* c, std::vector<double>& out5) {
     TRY(refresh_stage(c));
+    TRY(order_sources(c));
     EpiArgs ea;
     ea.mode = EPI_RHS;
     ea.omega = 2 * M_PI;
@@ -1149,6 +1221,7 @@ int fss_rhs_current(fss_ctx* c, double omega, double* modify5, double* psi) {
     if (!c->have) return fail(c, FSS_ERR_STATE, "no particles set");
     CU(cudaSetDevice(c->dev));
     TRY(refresh_stage(c));
+    TRY(order_sources(c));
     EpiArgs ea;
     ea.mode = EPI_RHS;
     ea.omega = omega;
@@ -1161,12 +1234,11 @@ int fss_rhs_current(fss_ctx* c, double omega, double* modify5, double* psi) {
 }
 
 namespace {
-// Pair evaluations the consumer lanes of a pair launch perform on items
-// [i0, i1) with `targets` consumer threads per block: per chunk of targets,
-// every full warp evaluates every source of the item (padded to whole
-// quads) on each lane; the last, partial warp (r targets) splits them over
-// 32 / r lanes per target, each lane taking every (32 / r)-th quad.
-double lane_pairs(const fss_ctx* c, int64_t i0, int64_t i1, int targets) {
+// Pair evaluations the lanes of a pair launch perform on items [i0, i1): every
+// 32 targets evaluate every source of the item (padded to whole quads) on
+// each lane; the last r targets split the sources over 32 / r lanes per
+// target, each lane taking every (32 / r)-th quad.
+double lane_pairs(const fss_ctx* c, int64_t i0, int64_t i1) {
     const ListOutput& L = c->lists;
     double sum = 0;
     for (int64_t i = i0; i < i1; i++) {
@@ -1178,11 +1250,8 @@ double lane_pairs(const fss_ctx* c, int64_t i0, int64_t i1, int targets) {
         }
         const double quads = std::ceil(src / 4.0);
         const int nt = it.leaf >= 0 ? c->leaf_start_h[it.leaf + 1] - c->leaf_start_h[it.leaf] : it.nt;
-        for (int c0 = 0; c0 < nt; c0 += targets) {
-            const int cn = std::min(targets, nt - c0);
-            sum += 32.0 * double(cn / 32) * 4.0 * quads;
-            if (cn % 32) sum += 32.0 * 4.0 * std::ceil(quads / double(32 / (cn % 32)));
-        }
+        sum += 32.0 * double(nt / 32) * 4.0 * quads;
+        if (nt % 32) sum += 32.0 * 4.0 * std::ceil(quads / double(32 / (nt % 32)));
     }
     return sum;
 }
@@ -1212,9 +1281,9 @@ int fss_get_tree_info(fss_ctx* c, fss_tree_info* info) {
     info->max_cluster_points = c->lists.down.empty() ? 0 : int32_t(c->lists.max_cluster_k);
     if (c->tree && c->have) {
         const int64_t nl = c->lists.n_leaf_items, na = int64_t(c->lists.items.size());
-        info->lane_pairs_leaf = lane_pairs(c, 0, nl, c->shape.targets());
+        info->lane_pairs_leaf = lane_pairs(c, 0, nl);
         if (na > nl)
-            info->lane_pairs_cluster = lane_pairs(c, nl, na, cluster_shape(c->fp64, c->lists.max_cluster_k).targets());
+            info->lane_pairs_cluster = lane_pairs(c, nl, na);
     }
     return FSS_OK;
 }
@@ -1453,6 +1522,7 @@ int fss_shard_stage(fss_ctx* c, int32_t stage, void* exchange) {
     if (stage == 1) {
         TRY(refresh_stage(c));
         if (c->tree && c->resort) TRY(resort(c));
+        TRY(order_sources(c));
     }
     bool down = false;
     TRY(eval_partials(c, false, &down));
@@ -1487,6 +1557,7 @@ int fss_shard_combine(fss_ctx* c, int32_t stage, double dt, double omega, const 
     ea.area = c->area_s.as<double>();
     ea.wtotal = c->wtotal.as<double>();
     ea.perm = c->tree ? c->perm.as<int32_t>() : nullptr;
+    ea.order = ordered(c) ? c->sortq.as<int32_t>() : nullptr;
     ea.src = c->src.p;
     ea.leaf_of = nullptr;
     ea.frame = nullptr;

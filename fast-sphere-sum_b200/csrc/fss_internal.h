@@ -31,7 +31,7 @@ struct Segment {
 };
 
 // One block's work.  leaf >= 0: the targets are that leaf's current
-// particles, taken in chunks of the block size; leaf < 0: the targets are
+// particles, taken in chunks (chunk_targets); leaf < 0: the targets are
 // [t0, t0 + nt).  Sources: segments [g0, g1).  Results go to partial slot
 // `part`.
 struct WorkItem {
@@ -40,6 +40,19 @@ struct WorkItem {
     int32_t part;
     int32_t leaf;
 };
+
+// Targets of a work item that one pass of a pair block serves: up to kMaxFull
+// a lane and a remainder of up to 31 more; more targets than that are taken
+// in chunks of near-equal size, at most 32 kMaxFull each.
+constexpr int kMaxFull = 4;
+constexpr int kChunkTargets = 32 * kMaxFull;
+FSS_HD inline int chunk_count(int nt) {
+    return nt < kChunkTargets + 32 ? (nt > 0 ? 1 : 0) : (nt + kChunkTargets - 1) / kChunkTargets;
+}
+FSS_HD inline int chunk_targets(int nt) {
+    const int chunks = chunk_count(nt);
+    return chunks <= 1 ? nt : (nt + chunks - 1) / chunks;
+}
 
 // Default limit of a bounded wait, in nanoseconds of %globaltimer (a context
 // can set its own).
@@ -55,8 +68,11 @@ struct PairCtl {
     int32_t pad;
 };
 
-// Sources per shared-memory tile: 256 float4 (4 KB) or 128 double4 (4 KB).
-FSS_HD constexpr int tile_capacity(bool fp64) { return fp64 ? 128 : 256; }
+// Sources per shared-memory tile: 256 float4 (4 KB) or 256 double4 (8 KB).
+FSS_HD constexpr int tile_capacity(bool fp64) {
+    (void)fp64;
+    return 256;
+}
 
 // Upward-pass combine work: node `node` (global index, levels concatenated)
 // on `level`; proxies of degree set `degmask` (bit d = degree d) written at

@@ -186,34 +186,35 @@ __global__ void k_epilogue(EpiArgs a) {
         const double4 v = a.partials[int64_t(p) * a.pstride + s];
         Ax += v.x; Ay += v.y; Az += v.z; Ap += v.w;
     }
-    const double4 x = a.xs[s];
+    const int64_t k = a.order ? a.order[s] : s;  // index in the state's order
+    const double4 x = a.xs[k];
     const double c = -1.0 / (2.0 * M_PI);
     const double ux = c * (x.y * Az - x.z * Ay);
     const double uy = c * (x.z * Ax - x.x * Az);
     const double uz = c * (x.x * Ay - x.y * Ax);
     const double dzeta = -2 * a.omega * uz;
     if (a.mode == EPI_RHS) {
-        const int64_t i = a.perm ? a.perm[s] : s;
+        const int64_t i = a.perm ? a.perm[k] : k;
         double* m = a.out5 + 5 * i;
         m[0] = ux; m[1] = uy; m[2] = uz; m[3] = dzeta; m[4] = 0.0 * (-1.0 / (4.0 * M_PI));
         if (a.psi) {
-            const double wself = x.w * a.area[s];
+            const double wself = x.w * a.area[k];
             a.psi[i] = -(M_LN2 / (4.0 * M_PI)) * (Ap - (a.wtotal[0] - wself));
         }
         return;
     }
-    const double4 s0 = a.s0[s];
+    const double4 s0 = a.s0[k];
     double4 acc;
     if (a.stage == 1) {
         acc = make_double4(ux, uy, uz, dzeta);
     } else {
         const double f = (a.stage == 4) ? 1.0 : 2.0;
-        acc = a.acc[s];
+        acc = a.acc[k];
         acc.x += ux * f; acc.y += uy * f; acc.z += uz * f; acc.w += dzeta * f;
     }
     double t[4];
     if (a.stage < 4) {
-        a.acc[s] = acc;
+        a.acc[k] = acc;
         const double h = (a.stage == 3) ? a.dt : a.dt / 2;
         t[0] = ux * h; t[1] = uy * h; t[2] = uz * h; t[3] = dzeta * h;
         t[0] += s0.x; t[1] += s0.y; t[2] += s0.z; t[3] += s0.w;
@@ -230,8 +231,8 @@ __global__ void k_epilogue(EpiArgs a) {
     const double px = t[0] * sc, py = t[1] * sc, pz = t[2] * sc;
     const double zeta = t[3] + (-2 * a.omega) * (pz - t[2]);
     const double4 nx = make_double4(px, py, pz, zeta);
-    if (a.stage == 4) a.s0[s] = nx;
-    a.xs[s] = nx;
+    if (a.stage == 4) a.s0[k] = nx;
+    a.xs[k] = nx;
     double fx = 0, fy = 0, fz = 0;
     if (a.frame && a.leaf_of) {
         const double4 f = a.frame[a.leaf_of[s]];
@@ -241,7 +242,7 @@ __global__ void k_epilogue(EpiArgs a) {
     o.x = T(px - fx);
     o.y = T(py - fy);
     o.z = T(pz - fz);
-    o.w = T(zeta * a.area[s]);
+    o.w = T(zeta * a.area[k]);
     static_cast<typename Vec4<T>::type*>(a.src)[s] = o;
 }
 

@@ -532,7 +532,7 @@ static cudaError_t run_pairs(cudaStream_t st, int nitems, const void* src, const
 
 const std::vector<PairShape>& pair_shapes(bool fp64) {
     static const std::vector<PairShape> f32 = {{160, 1, 256}, {192, 1, 256}, {224, 1, 256}, {288, 1, 256}};
-    static const std::vector<PairShape> f64 = {{160, 1, 128}, {192, 1, 128}, {224, 1, 128}, {288, 1, 128}};
+    static const std::vector<PairShape> f64 = {{160, 1, 256}, {192, 1, 256}, {224, 1, 256}, {288, 1, 256}};  // k_plane.cu
     return fp64 ? f64 : f32;
 }
 
@@ -544,6 +544,7 @@ PairShape pairs_shape(bool fp64, int threads, int per_thread) {
 }
 
 PairShape cluster_shape(bool fp64, int k) {
+    if (fp64) return pair_shapes(true).front();
     const int tile = tile_capacity(fp64);
     const int depth = kClusterDepth;
     if (k <= 32) return PairShape{64, 1, tile, depth};
@@ -582,9 +583,8 @@ cudaError_t launch_pairs(cudaStream_t st, bool fp64, bool psi, PairShape shape, 
                          const Segment* segs, const int32_t* leaf_start, const WorkItem* items,
                          double4* partials, int64_t pstride, int* err, PairCtl ctl) {
     if (fp64)
-        return psi ? dispatch<double, true>(st, shape, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl)
-                   : dispatch<double, false>(st, shape, nitems, src, segs, leaf_start, items, partials, pstride, err,
-                                             ctl);
+        return launch_plane_pairs(st, psi, shape.warps(), nitems, src, segs, leaf_start, items, partials, pstride, err,
+                                  ctl);
     return psi ? dispatch<float, true>(st, shape, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl)
                : dispatch<float, false>(st, shape, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
 }

@@ -34,16 +34,20 @@ struct EpiArgs {
     void* src = nullptr;
     const uint32_t* leaf_of = nullptr;
     const double4* frame = nullptr;
+    // FP64 direct sum: state index of each slot of partials and src (null: the same)
+    const int32_t* order = nullptr;
 };
 
-// Pair-kernel block: `threads` = one producer warp + consumer warps with one
-// target each.
+// Pair-kernel block.  FP32 (k_pairs.cu): one producer warp and consumer warps
+// with one target a thread.  FP64 (k_plane.cu): threads / 32 - 1 warps, which
+// share an item's sources.
 struct PairShape {
     int threads = 160;
     int per_thread = 1;
     int tile = 256;
     int depth = 4;  // ring slots (tiles in flight)
     int targets() const { return (threads - 32) * per_thread; }
+    int warps() const { return threads / 32 - 1; }
 };
 
 // k_tree.cu
@@ -76,14 +80,20 @@ void launch_resort_partition(cudaStream_t st, bool fp64, int64_t n, int64_t nlea
                              const NodeGeom* node, const int64_t* lev_off, uint32_t* key, uint32_t* key_new,
                              int32_t* leaf_start, int32_t* bucket, uint32_t* scratch, double4* s0, double* area,
                              double* tracer, int32_t* perm, double4* xs, double4* acc, void* src, int* err);
+// FP64 direct sum: the spatial order of the stage state's positions (order:
+// slot -> state index; key, key_tmp, vals_tmp n words each, hist as
+// launch_sort) and the sources in it.
+int order_launch_count(int64_t n);
+void launch_order(cudaStream_t st, int64_t n, const double4* xs, const double* area, uint32_t* key,
+                  uint32_t* key_tmp, int32_t* order, int32_t* vals_tmp, uint32_t* hist, double4* src);
 void launch_gather(cudaStream_t st, bool fp64, int64_t n, const double* in5, const double* area_in, const int32_t* perm,
                    const uint32_t* leaf_of, const double4* frame, double4* s0, double4* xs, double* area_s,
                    double* tracer_s, void* src);
 
 // k_pairs.cu
-// Block shapes of the pair kernel the autotuner tries (threads = 32 + targets).
+// Block shapes of the pair kernel the autotuner tries.
 const std::vector<PairShape>& pair_shapes(bool fp64);
-// The supported shape with `threads`, or the default (128).
+// The supported shape with `threads`, or the default (160).
 PairShape pairs_shape(bool fp64, int threads, int per_thread);
 // Block for work items of k targets (target clusters: their interpolation
 // points): the smallest of 64, 96, 128, 160 threads whose consumers hold them.
@@ -91,6 +101,10 @@ PairShape cluster_shape(bool fp64, int k);
 cudaError_t launch_pairs(cudaStream_t st, bool fp64, bool psi, PairShape shape, int nitems, const void* src,
                          const Segment* segs, const int32_t* leaf_start, const WorkItem* items, double4* partials,
                          int64_t pstride, int* err, PairCtl ctl);
+// The FP64 engine (k_plane.cu), launched by launch_pairs.
+cudaError_t launch_plane_pairs(cudaStream_t st, bool psi, int warps, int nitems, const void* src, const Segment* segs,
+                               const int32_t* leaf_start, const WorkItem* items, double4* partials, int64_t pstride,
+                               int* err, PairCtl ctl);
 constexpr int kPersistentThreads = 160;
 cudaError_t launch_pairs_persistent(cudaStream_t st, int nitems, const void* src, const Segment* segs,
                                     const int32_t* leaf_start, const WorkItem* items, int* queue, double4* partials,

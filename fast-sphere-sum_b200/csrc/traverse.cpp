@@ -247,7 +247,6 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
             if (a.proxy) need_slot(a.level, a.node, a.deg);
     }
     // segments and items
-    const int TB = in.threads * in.per_thread;
     const int P = std::max(1, in.parts);
     struct Cost { double cost; WorkItem it; };
     std::vector<Cost> items;
@@ -290,7 +289,7 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
                 if (acc >= total * p / P) cut[p++] = k + 1;
             }
         }
-        const int chunks = std::max(1, (nt_est + TB - 1) / TB);
+        const int chunks = std::max(1, chunk_count(nt_est));
         for (int p = 0; p < P; p++) {
             const int32_t base = int32_t(out.segs.size());
             double w = 0;
