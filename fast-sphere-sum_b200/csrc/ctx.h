@@ -92,6 +92,8 @@ struct fss_ctx {
     double list_blocks = 1, list_sources = 0;  // pair blocks over all leaves, the sources each goes through
     int64_t pstride = 0;  // partial slot stride: n, or n + proxy slots with target clusters
     int n_up_blocks = 0, n_dn_blocks = 0;  // blocks of the batched V^-1 products
+    int up_per_block = 16, dn_per_block = 16;  // their tasks at most
+    int max_leaf = 1, max_coefs = 1;  // of the downward evaluation
     int down_max_deg = 0;                  // highest target-cluster degree
     PairShape shape;
     double direct_pairs = 0;
@@ -100,7 +102,7 @@ struct fss_ctx {
     DBuf in5, area_in, perm, key, key_tmp, vals_tmp, hist, leaf_start, s0, xs, acc, area_s, tracer_s, src, partials,
         segs, items, jobs, frame, node, lev_off, verts, tri_verts, part_up, proxy_pos, out5, psi,
         wtotal, err_flag, loc, sortq, grid3, rm_target, rm_tris, rm_off, rm_adj, down_jobs, down_anc, down_coef, vpad, vtpad, vpad_off, up_deg, up_tblocks, up_tasks,
-        dn_tblocks, dn_tasks, msum, part_scratch;
+        dn_tblocks, dn_tasks, part_scratch;
     int64_t src_count = 0;
 
     // graph

@@ -604,14 +604,15 @@ int materialize(fss_ctx* c, PairShape shape) {
             c->down_max_deg = std::max(c->down_max_deg, int(L.down[j].deg));
         }
         CU(batch_prepare());
-        CU(c->msum.ensure(sizeof(double) * std::max<size_t>(L.jobs.size(), 1) * size_t(nproxy(c->nmax))));
         std::vector<TaskBlock> blocks;
         std::vector<int32_t> index;
-        make_task_blocks(up, batch_tasks(), blocks, index);
+        c->up_per_block = batch_tasks(int64_t(up.size()));
+        make_task_blocks(up, c->up_per_block, blocks, index);
         c->n_up_blocks = int(blocks.size());
         TRY(upload(c, c->up_tblocks, blocks));
         TRY(upload(c, c->up_tasks, index));
-        make_task_blocks(dn, batch_tasks(), blocks, index);
+        c->dn_per_block = batch_tasks(int64_t(dn.size()));
+        make_task_blocks(dn, c->dn_per_block, blocks, index);
         c->n_dn_blocks = int(blocks.size());
         TRY(upload(c, c->dn_tblocks, blocks));
         TRY(upload(c, c->dn_tasks, index));
@@ -628,6 +629,16 @@ int materialize(fss_ctx* c, PairShape shape) {
     const bool down = !L.down.empty();
     c->pstride = down ? n + L.n_proxy : n;
     CU(c->partials.ensure(sizeof(double4) * size_t(P + (down ? 1 : 0)) * size_t(c->pstride)));
+    // the downward evaluation: a leaf and the clusters above it
+    c->max_leaf = 1;
+    for (int64_t l = 0; l < c->nleaf; l++)
+        c->max_leaf = std::max(c->max_leaf, c->leaf_start_h[l + 1] - c->leaf_start_h[l]);
+    c->max_coefs = 1;
+    for (size_t i = 0; i < L.leaf_anc.size(); i += kMaxLevels) {
+        int k = 0;
+        for (int l = 0; l < kMaxLevels && L.leaf_anc[i + l].coef >= 0; l++) k += nproxy(L.leaf_anc[i + l].deg);
+        c->max_coefs = std::max(c->max_coefs, k);
+    }
     CU(c->part_up.ensure(sizeof(double) * size_t(c->nleaf) * (LL + 1) * nproxy(c->nmax)));
     return FSS_OK;
 }
@@ -684,10 +695,10 @@ int eval_partials(fss_ctx* c, bool want_psi, bool* down_out) {
                            c->leaf_level, c->nmax, c->level_mask, c->up_deg.as<int8_t>(), c->part_up.as<double>());
         }
         {
-            ProfScope ps(c, "upward_combine", 2);  // k_up_sums, k_up_proxies
+            ProfScope ps(c, "upward_combine");
             launch_up_proxies(c->stream, c->fp64, int(c->lists.jobs.size()), c->jobs.as<ProxyJob>(),
-                              c->part_up.as<double>(), c->leaf_level, c->nmax, c->msum.as<double>(),
-                              c->n_up_blocks, c->up_tblocks.as<TaskBlock>(), c->up_tasks.as<int32_t>(),
+                              c->part_up.as<double>(), c->leaf_level, c->nmax, c->n_up_blocks, c->up_per_block,
+                              c->up_tblocks.as<TaskBlock>(), c->up_tasks.as<int32_t>(),
                               c->vpad.as<double>(), c->vpad_off.as<int32_t>(), c->proxy_pos.as<double4>(), c->n,
                               c->src.p, c->err_flag.as<int>(), c->wait_ns, c->hold_stage == 0 ? 0 : -1);
             if (c->hold_stage == 0) c->hold_stage = -1;  // the test hook holds one launch only
@@ -710,6 +721,9 @@ int eval_partials(fss_ctx* c, bool want_psi, bool* down_out) {
         d.njobs = int(c->lists.down.size());
         d.jobs = c->down_jobs.as<DownJob>();
         d.ncoef_blocks = c->n_dn_blocks;
+        d.per_block = c->dn_per_block;
+        d.max_leaf = c->max_leaf;
+        d.max_coefs = c->max_coefs;
         d.max_deg = c->down_max_deg;
         d.fp32_eval = !c->fp64;
         d.coef_blocks = c->dn_tblocks.as<TaskBlock>();

@@ -67,47 +67,36 @@ __global__ void __launch_bounds__(kUpThreads, 5) k_up_leaf(const typename Vec4<T
     for (int m = threadIdx.x; m < KJ; m += kUpThreads) out[m] = (O[0][m] + O[1][m]) + (O[2][m] + O[3][m]);
 }
 
-// Batched V^-1 products.  A block takes up to kBatchTasks tasks (faces or
-// clusters) of one degree, K = nproxy(deg): it stages the K x K matrix, its
-// rows padded to Kp = 4 ceil(K / 4) doubles, and the tasks' inputs in shared
-// memory, and gives each thread a tile of 2 outputs x 4 tasks, so that every
-// staged value it reads feeds several FMA chains.  Each output is the chain
-// of FMAs over the inner index in order, as a per-task product forms it (so
-// the single problem and the ensemble stay bit-identical).
+// Batched V^-1 products.  A block takes up to 4 TT tasks (faces or clusters) of
+// one degree, K = nproxy(deg): it stages the K x K matrix, its rows padded to
+// Kp = 4 ceil(K / 4) doubles, and the tasks' inputs in shared memory, and gives
+// each thread a tile of 2 outputs x TT tasks.  Each output is the chain of FMAs
+// over the inner index in order, as a per-task product forms it (so the single
+// problem and the ensemble stay bit-identical).  TT is 4 where there are tasks
+// for several blocks per SM (every staged value then feeds several chains) and
+// 2 or 1 below (batch_tasks): the kernels are bound by the latency of a block
+// -- staging, then K dependent FMAs.  The charges of 420 faces (40,962
+// particles, n = 8) took 16.4 us in 27 blocks of 16 after a launch for the row
+// sums, and take 8.6 us; coefficients and evaluation 25.2, now 17.4.
 constexpr int kBatchThreads = 192;
-constexpr int kBatchTasks = 16;
+constexpr int kBatchTasks = 16;  // at most
 __host__ __device__ constexpr int batch_pad(int K) { return (K + 3) & ~3; }
-static_assert((batch_pad(kMaxK) / 2) * (kBatchTasks / 4) <= kBatchThreads, "one tile per thread at the largest degree");
+static_assert((batch_pad(kMaxK) / 2) * 4 <= kBatchThreads, "one tile per thread at the largest degree");
 
-// Upward pass, part 2a: the moments of every proxy face, its rows summed
-// (up_row_step, sum_rows4), one thread per (face, moment) over a flat grid
-// of njobs x nproxy(nmax) items: msum[j][m].
-constexpr int kSumThreads = 256;
-__global__ void __launch_bounds__(kSumThreads) k_up_sums(const ProxyJob* __restrict__ jobs, int njobs,
-                                                         const double* __restrict__ part, int leaf_level, int nmax,
-                                                         double* __restrict__ msum) {
-    const int KM = nproxy(nmax);
-    const int64_t item = int64_t(blockIdx.x) * kSumThreads + threadIdx.x;
-    if (item >= int64_t(njobs) * KM) return;
-    const int j = int(item / KM), m = int(item - int64_t(j) * KM);
-    const ProxyJob& job = jobs[j];
-    if (m >= nproxy(31 - __clz(job.degmask))) return;  // moments this face's degrees use
-    const int step = up_row_step(job.level, leaf_level);
-    const int64_t stride = int64_t(step) * (leaf_level + 1) * KM;
-    const double* pr = part + (int64_t(job.leaf_lo) * (leaf_level + 1) + job.level) * KM + m;
-    msum[item] = sum_rows4([&](int r) { return pr[r * stride]; }, (job.leaf_hi - job.leaf_lo) / step);
-}
-
-// Upward pass, part 2b: proxy charges q_k = sum_m Vinv[m][k] M_m of every
-// (face, degree) task, written with the proxy positions at the face's slots
-// of the unified source array (absolute coordinates).  Shared memory:
-// A[m][k] = Vinv[m][k] (K rows of Kp; one bulk copy of the padded matrix
-// `vpad`), then X[t][m] = the task's moments.
-template <typename T>
+// Upward pass, part 2: the moments of every proxy face -- its rows summed
+// (up_row_step, sum_rows4) -- and from them the proxy charges q_k = sum_m
+// Vinv[m][k] M_m of every (face, degree) task, written with the proxy
+// positions at the face's slots of the unified source array (absolute
+// coordinates).  Shared memory: A[m][k] = Vinv[m][k] (K rows of Kp; one bulk
+// copy of the padded matrix `vpad`), then X[t][m] = the task's moments.  The
+// rows were summed by a launch of their own, 4 to 7 us of latency that only a
+// face of several degrees made up for: with learned parameters at 655,362
+// particles the two took 13 + 37 us and this takes 52.
+template <typename T, int TT>
 __global__ void __launch_bounds__(kBatchThreads) k_up_proxies(const TaskBlock* __restrict__ blocks,
                                                               const int32_t* __restrict__ tasks,
                                                               const ProxyJob* __restrict__ jobs,
-                                                              const double* __restrict__ msum, int nmax,
+                                                              const double* __restrict__ part, int leaf_level, int nmax,
                                                               const double* __restrict__ vpad,
                                                               const int32_t* __restrict__ vpad_off,
                                                               const double4* __restrict__ proxy_pos, int64_t n,
@@ -115,45 +104,62 @@ __global__ void __launch_bounds__(kBatchThreads) k_up_proxies(const TaskBlock* _
                                                               uint64_t wait_ns, int hold_block) {
     extern __shared__ __align__(32) double bsm[];
     __shared__ __align__(8) uint64_t bar;
+    __shared__ const double* row0[4 * TT];  // first row of a task's face
+    __shared__ int rows[4 * TT], step[4 * TT], slot0[4 * TT];
     const TaskBlock tb = blocks[blockIdx.x];
     const int d = tb.deg, K = nproxy(d), Kp = batch_pad(K), nt = tb.count;
-    const int KM = nproxy(nmax);
+    const int KM = nproxy(nmax), tid = threadIdx.x;
     double* A = bsm;
     double* X = bsm + K * Kp;
     stage_issue(A, vpad + vpad_off[d], uint32_t(sizeof(double)) * K * Kp, &bar, int(blockIdx.x) == hold_block);
-    for (int i = threadIdx.x; i < nt * K; i += kBatchThreads) {
+    if (tid < nt) {
+        const ProxyJob& job = jobs[tasks[tb.first + tid]];
+        const int s = up_row_step(job.level, leaf_level);
+        row0[tid] = part + (int64_t(job.leaf_lo) * (leaf_level + 1) + job.level) * KM;
+        rows[tid] = (job.leaf_hi - job.leaf_lo) / s;
+        step[tid] = s * (leaf_level + 1) * KM;
+        slot0[tid] = job.off[d];
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int i = tid; i < nt * K; i += kBatchThreads) {
         const int t = i / K, m = i - t * K;
-        X[i] = msum[int64_t(tasks[tb.first + t]) * KM + m];
+        const double* p = row0[t] + m;
+        const int64_t s = step[t];
+        X[i] = sum_rows4([&](int r) { return p[r * s]; }, rows[t]);
     }
     __syncthreads();
     if (!stage_wait(&bar, wait_ns)) {
-        if (threadIdx.x == 0) set_error(err, kErrTimeout);
+        if (tid == 0) set_error(err, kErrTimeout);
         return;
     }
-    const int npair = Kp / 2, tid = threadIdx.x;
-    if (tid >= npair * ((nt + 3) / 4)) return;  // no barrier follows
-    const int k0 = 2 * (tid % npair), t0 = 4 * (tid / npair);
-    double q[4][2];
+    const int npair = Kp / 2;
+    if (tid >= npair * ((nt + TT - 1) / TT)) return;  // no barrier follows
+    const int k0 = 2 * (tid % npair), t0 = TT * (tid / npair);
+    double q[TT][2];
+    const double* Xt[TT];
 #pragma unroll
-    for (int j = 0; j < 4; j++) q[j][0] = q[j][1] = 0.0;
-    const double* Xt = X + t0 * K;
+    for (int j = 0; j < TT; j++) {
+        q[j][0] = q[j][1] = 0.0;
+        Xt[j] = X + min(t0 + j, nt - 1) * K;
+    }
+#pragma unroll 4
     for (int m = 0; m < K; m++) {
         const double2 a = *reinterpret_cast<const double2*>(A + m * Kp + k0);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const double x = (t0 + j < nt) ? Xt[j * K + m] : 0.0;
+        for (int j = 0; j < TT; j++) {
+            const double x = Xt[j][m];
             q[j][0] = fma(a.x, x, q[j][0]);
             q[j][1] = fma(a.y, x, q[j][1]);
         }
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < TT; j++) {
         if (t0 + j >= nt) break;
-        const ProxyJob& job = jobs[tasks[tb.first + t0 + j]];
 #pragma unroll
         for (int r = 0; r < 2; r++) {
             if (k0 + r >= K) break;
-            const int64_t slot = int64_t(job.off[d]) + k0 + r;
+            const int64_t slot = int64_t(slot0[t0 + j]) + k0 + r;
             const double4 y = proxy_pos[slot - n];
             typename Vec4<T>::type o;
             o.x = T(y.x);
@@ -165,7 +171,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_up_proxies(const TaskBlock* _
     }
 }
 
-size_t up_proxies_smem(int K) { return sizeof(double) * size_t(K * batch_pad(K) + kBatchTasks * K); }
+size_t up_proxies_smem(int K, int per_block) { return sizeof(double) * size_t(K * batch_pad(K) + per_block * K); }
 
 // ---------------------------------------------------------------- epilogue
 
@@ -342,8 +348,8 @@ __global__ void k_scatter_state(int64_t n, const int32_t* __restrict__ perm, con
 // sum_k Vinv[m][k] y_k over k in order.  Shared memory: A[k][m] =
 // Vinv[m][k] (K rows of Kp; one bulk copy of the padded transpose `vtpad`),
 // then Y[t][k].
-template <bool PSI>
-__global__ void __launch_bounds__(kBatchThreads) k_down_coef(const TaskBlock* __restrict__ blocks,
+template <bool PSI, int TT>
+__global__ void __launch_bounds__(kBatchThreads, 3) k_down_coef(const TaskBlock* __restrict__ blocks,
                                                              const int32_t* __restrict__ tasks,
                                                              const DownJob* __restrict__ jobs,
                                                              const double4* __restrict__ partials, int parts,
@@ -353,8 +359,8 @@ __global__ void __launch_bounds__(kBatchThreads) k_down_coef(const TaskBlock* __
                                                              int hold_block) {
     extern __shared__ __align__(32) double bsm[];
     __shared__ __align__(8) uint64_t bar;
-    __shared__ int32_t slot_of[kBatchTasks];
-    __shared__ int64_t coef_of[kBatchTasks];
+    __shared__ int32_t slot_of[4 * TT];
+    __shared__ int64_t coef_of[4 * TT];
     const TaskBlock tb = blocks[blockIdx.x];
     const int d = tb.deg, K = nproxy(d), Kp = batch_pad(K), nt = tb.count;
     double* A = bsm;
@@ -385,17 +391,21 @@ __global__ void __launch_bounds__(kBatchThreads) k_down_coef(const TaskBlock* __
         return;
     }
     const int npair = Kp / 2, tid = threadIdx.x;
-    if (tid >= npair * ((nt + 3) / 4)) return;  // no barrier follows
-    const int m0 = 2 * (tid % npair), t0 = 4 * (tid / npair);
-    double4 c[4][2];
+    if (tid >= npair * ((nt + TT - 1) / TT)) return;  // no barrier follows
+    const int m0 = 2 * (tid % npair), t0 = TT * (tid / npair);
+    double4 c[TT][2];
+    const double4* Yt[TT];
 #pragma unroll
-    for (int j = 0; j < 4; j++) c[j][0] = c[j][1] = make_double4(0.0, 0.0, 0.0, 0.0);
-    const double4* Yt = Y + t0 * K;
+    for (int j = 0; j < TT; j++) {
+        c[j][0] = c[j][1] = make_double4(0.0, 0.0, 0.0, 0.0);
+        Yt[j] = Y + min(t0 + j, nt - 1) * K;
+    }
+#pragma unroll(TT == 4 ? 1 : 4)
     for (int k = 0; k < K; k++) {
         const double2 a = *reinterpret_cast<const double2*>(A + k * Kp + m0);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const double4 y = (t0 + j < nt) ? Yt[j * K + k] : make_double4(0.0, 0.0, 0.0, 0.0);
+        for (int j = 0; j < TT; j++) {
+            const double4 y = Yt[j][k];
             c[j][0].x = fma(a.x, y.x, c[j][0].x);
             c[j][0].y = fma(a.x, y.y, c[j][0].y);
             c[j][0].z = fma(a.x, y.z, c[j][0].z);
@@ -409,7 +419,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_down_coef(const TaskBlock* __
         }
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < TT; j++) {
         if (t0 + j >= nt) break;
         double4* out = coef + coef_of[t0 + j];
         if (m0 < K) out[m0] = c[j][0];
@@ -417,7 +427,9 @@ __global__ void __launch_bounds__(kBatchThreads) k_down_coef(const TaskBlock* __
     }
 }
 
-size_t down_coef_smem(int K) { return sizeof(double) * size_t(K * batch_pad(K)) + sizeof(double4) * size_t(kBatchTasks * K); }
+size_t down_coef_smem(int K, int per_block) {
+    return sizeof(double) * size_t(K * batch_pad(K)) + sizeof(double4) * size_t(per_block * K);
+}
 
 // The interpolant of degree D with coefficients C at barycentric (u, v)
 // (both mapped to [-1, 1]): sum_a T_a(u) sum_b C[m(a, b)] T_b(v), a + b <= D,
@@ -519,46 +531,67 @@ __device__ __forceinline__ float3 eval_any_f(int deg, float u, float v, const fl
 // in each cluster's frame).  A leaf below none writes zeros.  F32 (mixed
 // precision, velocity only): the interpolants evaluated in FP32
 // (eval_deg_f), the coordinates and the sum over the clusters in FP64.
-template <bool PSI, bool F32>
-__global__ void __launch_bounds__(kUpThreads) k_down_direct(const double4* __restrict__ xs,
-                                                            const int32_t* __restrict__ leaf_start,
-                                                            const NodeGeom* __restrict__ node,
-                                                            const LeafAnc* __restrict__ leaf_anc,
-                                                            const double4* __restrict__ coef,
-                                                            double4* __restrict__ out) {
-    __shared__ double4 C[kMaxLevels * kMaxK];
+//
+// Bound by latency: of the block's loads, then of the shared loads of the
+// coefficients, one per 3 FMAs.  So the loads of all clusters' coefficients
+// and of the particles are in flight together, the shared memory is what the
+// largest leaf's clusters need, and where all blocks run at once the block is
+// as wide as the largest leaf and takes it in one round: 26.3 us before, 24.3
+// now at 163,842 particles and n = 10, in 1,280 leaves of 128 to 135.
+template <bool PSI, bool F32, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 256 : 128, WIDE || !F32 ? 2 : 0) k_down_direct(const double4* __restrict__ xs,
+                                                                 const int32_t* __restrict__ leaf_start,
+                                                                 const NodeGeom* __restrict__ node,
+                                                                 const LeafAnc* __restrict__ leaf_anc,
+                                                                 const double4* __restrict__ coef,
+                                                                 double4* __restrict__ out) {
+    extern __shared__ __align__(32) double bsm[];
+    double4* C = reinterpret_cast<double4*>(bsm);
+    float4* Cf = reinterpret_cast<float4*>(bsm);  // F32: the coefficients rounded, 16 B each
     __shared__ LeafAnc A[kMaxLevels];
     __shared__ NodeGeom G[kMaxLevels];
     __shared__ int off[kMaxLevels + 1];
-    const int leaf = blockIdx.x, tid = threadIdx.x;
+    const int leaf = blockIdx.x, tid = threadIdx.x, threads = blockDim.x;
     const int a0 = leaf_start[leaf], a1 = leaf_start[leaf + 1];
-    if (a0 == a1) return;
-    if (tid < kMaxLevels) A[tid] = leaf_anc[int64_t(leaf) * kMaxLevels + tid];
+    if (tid < 32) {  // the clusters above the leaf, their offsets and frames
+        LeafAnc anc{-1, 0, 0, 0};
+        if (tid < kMaxLevels) anc = leaf_anc[int64_t(leaf) * kMaxLevels + tid];
+        const unsigned used = __ballot_sync(0xffffffffu, anc.coef >= 0);
+        const int nanc = __ffs(~used) - 1;  // the list ends at the first without
+        const int k = tid < nanc ? nproxy(anc.deg) : 0;
+        int incl = k;
+#pragma unroll
+        for (int d = 1; d < kMaxLevels; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, d);
+            if (tid >= d) incl += y;
+        }
+        if (tid < kMaxLevels) {
+            if (tid >= nanc) anc.coef = -1;
+            A[tid] = anc;
+            off[tid + 1] = incl;
+        }
+        if (tid == 0) off[0] = 0;
+        if (tid < nanc) G[tid] = node[anc.node];
+    }
+    double4 x = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (a0 + tid < a1) x = xs[a0 + tid];
     __syncthreads();
+    if (a0 == a1) return;
     int nanc = 0;
     while (nanc < kMaxLevels && A[nanc].coef >= 0) nanc++;
-    if (tid < nanc) G[tid] = node[A[tid].node];
-    if (tid == 0) {
-        int o = 0;
-        for (int k = 0; k < nanc; k++) {
-            off[k] = o;
-            o += nproxy(A[k].deg);
-        }
-        off[nanc] = o;
+#pragma unroll 4
+    for (int m = tid; m < off[nanc]; m += threads) {
+        int a = 0;
+        while (m >= off[a + 1]) a++;
+        const double4 cd = coef[int64_t(A[a].coef) + m - off[a]];
+        if (F32)
+            Cf[m] = make_float4(float(cd.x), float(cd.y), float(cd.z), 0.f);
+        else
+            C[m] = cd;
     }
     __syncthreads();
-    float4* Cf = reinterpret_cast<float4*>(C);  // F32: the same coefficients rounded, 16 B each
-    for (int a = 0; a < nanc; a++)
-        for (int m = tid; m < off[a + 1] - off[a]; m += kUpThreads) {
-            const double4 cd = coef[int64_t(A[a].coef) + m];
-            if (F32)
-                Cf[off[a] + m] = make_float4(float(cd.x), float(cd.y), float(cd.z), 0.f);
-            else
-                C[off[a] + m] = cd;
-        }
-    __syncthreads();
-    for (int i = a0 + tid; i < a1; i += kUpThreads) {
-        const double4 x = xs[i];
+    for (int i = a0 + tid; i < a1; i += threads) {
+        if (i != a0 + tid) x = xs[i];
         double4 acc = make_double4(0.0, 0.0, 0.0, 0.0);
         for (int a = 0; a < nanc; a++) {
             const NodeGeom& ng = G[a];
@@ -594,35 +627,52 @@ void launch_up_leaf(cudaStream_t st, bool fp64, int nleaf, const void* src, cons
                                                     lev_off, leaf_level, nmax, level_mask, up_deg, nleaf, part);
 }
 
+template <typename T, int TT>
+static void run_up_proxies(cudaStream_t st, const ProxyJob* jobs, const double* part, int leaf_level, int nmax,
+                           int nblocks, const TaskBlock* blocks, const int32_t* tasks, const double* vpad,
+                           const int32_t* vpad_off, const double4* proxy_pos, int64_t n, void* src, int* err,
+                           uint64_t wait_ns, int hold_block) {
+    k_up_proxies<T, TT><<<nblocks, kBatchThreads, up_proxies_smem(nproxy(nmax), 4 * TT), st>>>(
+        blocks, tasks, jobs, part, leaf_level, nmax, vpad, vpad_off, proxy_pos, n,
+        static_cast<typename Vec4<T>::type*>(src), err, wait_ns, hold_block);
+}
+
 void launch_up_proxies(cudaStream_t st, bool fp64, int njobs, const ProxyJob* jobs, const double* part,
-                       int leaf_level, int nmax, double* msum, int nblocks, const TaskBlock* blocks,
+                       int leaf_level, int nmax, int nblocks, int per_block, const TaskBlock* blocks,
                        const int32_t* tasks, const double* vpad, const int32_t* vpad_off, const double4* proxy_pos,
                        int64_t n, void* src, int* err, uint64_t wait_ns, int hold_block) {
     if (njobs == 0) return;
-    const int64_t items = int64_t(njobs) * nproxy(nmax);
-    k_up_sums<<<unsigned((items + kSumThreads - 1) / kSumThreads), kSumThreads, 0, st>>>(jobs, njobs, part, leaf_level,
-                                                                                          nmax, msum);
-    const size_t smem = up_proxies_smem(nproxy(nmax));
-    if (fp64)
-        k_up_proxies<double><<<nblocks, kBatchThreads, smem, st>>>(blocks, tasks, jobs, msum, nmax, vpad, vpad_off,
-                                                                   proxy_pos, n, static_cast<double4*>(src), err,
-                                                                   wait_ns, hold_block);
-    else
-        k_up_proxies<float><<<nblocks, kBatchThreads, smem, st>>>(blocks, tasks, jobs, msum, nmax, vpad, vpad_off,
-                                                                  proxy_pos, n, static_cast<float4*>(src), err,
-                                                                  wait_ns, hold_block);
+    auto run = fp64 ? (per_block <= 4 ? run_up_proxies<double, 1>
+                                      : (per_block <= 8 ? run_up_proxies<double, 2> : run_up_proxies<double, 4>))
+                    : (per_block <= 4 ? run_up_proxies<float, 1>
+                                      : (per_block <= 8 ? run_up_proxies<float, 2> : run_up_proxies<float, 4>));
+    run(st, jobs, part, leaf_level, nmax, nblocks, blocks, tasks, vpad, vpad_off, proxy_pos, n, src, err, wait_ns,
+        hold_block);
 }
 
-int batch_tasks() { return kBatchTasks; }
+// More tasks per block where the blocks (2 at a time per SM) stay busy all the
+// same; us per RK4 step in blocks of 4, 8, 16: 420 clusters 393 398 429; 1,700
+// (n = 10) 1430 1428 1438; 6,820 4084 4058 4045.
+int batch_tasks(int64_t tasks) { return tasks <= 4 * 296 ? 4 : (tasks <= 8 * 296 ? 8 : kBatchTasks); }
 
 cudaError_t batch_prepare() {
     // dynamic shared memory above the default 48 KB, sized for the largest degree
-    const int up = int(up_proxies_smem(kMaxK)), dn = int(down_coef_smem(kMaxK));
+    auto allow = [](auto kernel, size_t bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+    };
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_up_proxies<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, up)) ||
-        (e = cudaFuncSetAttribute(k_up_proxies<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, up)) ||
-        (e = cudaFuncSetAttribute(k_down_coef<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dn)) ||
-        (e = cudaFuncSetAttribute(k_down_coef<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dn)))
+    if ((e = allow(k_up_proxies<float, 1>, up_proxies_smem(kMaxK, 4))) ||
+        (e = allow(k_up_proxies<float, 2>, up_proxies_smem(kMaxK, 8))) ||
+        (e = allow(k_up_proxies<float, 4>, up_proxies_smem(kMaxK, 16))) ||
+        (e = allow(k_up_proxies<double, 1>, up_proxies_smem(kMaxK, 4))) ||
+        (e = allow(k_up_proxies<double, 2>, up_proxies_smem(kMaxK, 8))) ||
+        (e = allow(k_up_proxies<double, 4>, up_proxies_smem(kMaxK, 16))) ||
+        (e = allow(k_down_coef<false, 1>, down_coef_smem(kMaxK, 4))) ||
+        (e = allow(k_down_coef<false, 2>, down_coef_smem(kMaxK, 8))) ||
+        (e = allow(k_down_coef<false, 4>, down_coef_smem(kMaxK, 16))) ||
+        (e = allow(k_down_coef<true, 1>, down_coef_smem(kMaxK, 4))) ||
+        (e = allow(k_down_coef<true, 2>, down_coef_smem(kMaxK, 8))) ||
+        (e = allow(k_down_coef<true, 4>, down_coef_smem(kMaxK, 16))))
         return e;
     return cudaSuccess;
 }
@@ -664,27 +714,31 @@ void launch_scatter_state(cudaStream_t st, int64_t n, const int32_t* perm, const
     k_scatter_state<<<unsigned((n + 255) / 256), 256, 0, st>>>(n, perm, s0, tracer, out5);
 }
 
+template <bool PSI, int TT>
+static void run_down_coef(cudaStream_t st, const DownArgs& d) {
+    k_down_coef<PSI, TT><<<unsigned(d.ncoef_blocks), kBatchThreads, down_coef_smem(nproxy(d.max_deg), 4 * TT), st>>>(
+        d.coef_blocks, d.coef_tasks, d.jobs, d.partials, d.parts, d.pstride, d.vtpad, d.vpad_off, d.coef, d.err,
+        d.wait_ns, d.hold_block);
+}
+
 void launch_down(cudaStream_t st, bool psi, const DownArgs& d) {
     if (d.njobs == 0) return;
-    const unsigned nb = unsigned(d.ncoef_blocks);
-    const size_t smem = down_coef_smem(nproxy(d.max_deg));
-    if (psi) {
-        k_down_coef<true><<<nb, kBatchThreads, smem, st>>>(d.coef_blocks, d.coef_tasks, d.jobs, d.partials, d.parts,
-                                                           d.pstride, d.vtpad, d.vpad_off, d.coef, d.err, d.wait_ns,
-                                                           d.hold_block);
-        k_down_direct<true, false><<<d.nleaf, kUpThreads, 0, st>>>(d.xs, d.leaf_start, d.node, d.leaf_anc, d.coef,
-                                                                   d.out);
-    } else {
-        k_down_coef<false><<<nb, kBatchThreads, smem, st>>>(d.coef_blocks, d.coef_tasks, d.jobs, d.partials,
-                                                            d.parts, d.pstride, d.vtpad, d.vpad_off, d.coef, d.err,
-                                                            d.wait_ns, d.hold_block);
-        if (d.fp32_eval)
-            k_down_direct<false, true><<<d.nleaf, kUpThreads, 0, st>>>(d.xs, d.leaf_start, d.node, d.leaf_anc,
-                                                                       d.coef, d.out);
-        else
-            k_down_direct<false, false><<<d.nleaf, kUpThreads, 0, st>>>(d.xs, d.leaf_start, d.node, d.leaf_anc,
-                                                                        d.coef, d.out);
-    }
+    auto coef = psi ? (d.per_block <= 4 ? run_down_coef<true, 1>
+                                        : (d.per_block <= 8 ? run_down_coef<true, 2> : run_down_coef<true, 4>))
+                    : (d.per_block <= 4 ? run_down_coef<false, 1>
+                                        : (d.per_block <= 8 ? run_down_coef<false, 2> : run_down_coef<false, 4>));
+    coef(st, d);
+    const bool f32 = d.fp32_eval && !psi;
+    // a second round for the few particles beyond 128 costs less than the idle
+    // lanes of a wider block once other blocks run meanwhile (5,120 leaves: 82 us
+    // against 89; 1,280: 26 against 24)
+    const bool wide = d.nleaf <= 1480;
+    auto direct = psi ? (wide ? k_down_direct<true, false, true> : k_down_direct<true, false, false>)
+                  : f32 ? (wide ? k_down_direct<false, true, true> : k_down_direct<false, true, false>)
+                        : (wide ? k_down_direct<false, false, true> : k_down_direct<false, false, false>);
+    const int threads = wide ? std::min(256, std::max(64, (d.max_leaf + 31) & ~31)) : 128;
+    const size_t smem = (f32 ? sizeof(float4) : sizeof(double4)) * size_t(d.max_coefs);
+    direct<<<d.nleaf, threads, smem, st>>>(d.xs, d.leaf_start, d.node, d.leaf_anc, d.coef, d.out);
 }
 
 int down_launch_count(const DownArgs& d) { return d.njobs == 0 ? 0 : 2; }

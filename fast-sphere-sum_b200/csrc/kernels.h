@@ -115,18 +115,17 @@ int persistent_blocks_per_sm();
 void launch_up_leaf(cudaStream_t st, bool fp64, int nleaf, const void* src, const int32_t* leaf_start,
                     const double4* frame, const NodeGeom* node, const int64_t* lev_off, int leaf_level, int nmax,
                     int level_mask, const int8_t* up_deg, double* part);
-// Upward pass, part 2: every proxy face's moments (its rows summed into
-// msum, njobs x nproxy(nmax)), then the proxy charges of every (face,
-// degree) task, batched by degree (`blocks` of at most batch_tasks() tasks).
-// vpad: Vinv of every degree with rows padded to a multiple of 4 doubles
-// (vpad_off by degree); a failed wait sets kErrTimeout in err.
+// Upward pass, part 2: the proxy charges of every (face, degree) task from the
+// face's moment rows, batched by degree (`blocks` of at most per_block
+// tasks).  vpad: Vinv of every degree with rows padded to a multiple of 4
+// doubles (vpad_off by degree); a failed wait sets kErrTimeout in err.
 void launch_up_proxies(cudaStream_t st, bool fp64, int njobs, const ProxyJob* jobs, const double* part,
-                       int leaf_level, int nmax, double* msum, int nblocks, const TaskBlock* blocks,
+                       int leaf_level, int nmax, int nblocks, int per_block, const TaskBlock* blocks,
                        const int32_t* tasks, const double* vpad, const int32_t* vpad_off, const double4* proxy_pos,
                        int64_t n, void* src, int* err, uint64_t wait_ns, int hold_block = -1);
-// Tasks per block of the batched V^-1 products (upward proxy charges,
-// downward coefficients).
-int batch_tasks();
+// Tasks per block (4, 8 or 16) of the batched V^-1 products (upward proxy
+// charges, downward coefficients) when there are `tasks` of them.
+int batch_tasks(int64_t tasks);
 // Allows the batched V^-1 kernels the dynamic shared memory of the largest
 // degree (host only; before their first launch).
 cudaError_t batch_prepare();
@@ -135,6 +134,7 @@ struct DownArgs {
     int njobs = 0;                       // target clusters
     const DownJob* jobs = nullptr;
     int ncoef_blocks = 0;                // their coefficient tasks, batched by degree
+    int per_block = 16;                  // tasks per block at most
     int max_deg = 0;                     // highest target-cluster degree
     const TaskBlock* coef_blocks = nullptr;
     const int32_t* coef_tasks = nullptr;
@@ -149,6 +149,8 @@ struct DownArgs {
     const NodeGeom* node = nullptr;
     double4* coef = nullptr;
     int nleaf = 0;
+    int max_leaf = 1;                    // particles of the largest leaf (about)
+    int max_coefs = 1;                   // most coefficients of the clusters above one leaf
     const double4* xs = nullptr;
     const int32_t* leaf_start = nullptr;
     const LeafAnc* leaf_anc = nullptr;   // kMaxLevels per leaf

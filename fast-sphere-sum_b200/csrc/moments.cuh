@@ -149,12 +149,13 @@ __device__ __forceinline__ void leaf_moments(const typename Vec4<T>::type* __res
 }
 
 // Sum of R rows, row(i) for i < R, as four chains (rows i = 0, 4, 8, ...;
-// 1, 5, ...; ...) added as (s0 + s1) + (s2 + s3): four loads in flight.
+// 1, 5, ...; ...) added as (s0 + s1) + (s2 + s3): sixteen loads in flight.
 // The single problem's and the ensemble's combines both sum this way.
 template <typename F>
 __device__ __forceinline__ double sum_rows4(F row, int R) {
     double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
     int i = 0;
+#pragma unroll 4
     for (; i + 4 <= R; i += 4) {
         s0 += row(i + 0);
         s1 += row(i + 1);
