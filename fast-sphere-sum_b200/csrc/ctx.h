@@ -90,6 +90,7 @@ struct fss_ctx {
     int nmax = 0, level_mask = 0;
     int parts = 1;
     double list_blocks = 1, list_sources = 0;  // pair blocks over all leaves, the sources each goes through
+    bool member = false;  // of an ensemble: its items are whole leaves
     int64_t pstride = 0;  // partial slot stride: n, or n + proxy slots with target clusters
     int n_up_blocks = 0, n_dn_blocks = 0;  // blocks of the batched V^-1 products
     int up_per_block = 16, dn_per_block = 16;  // their tasks at most

@@ -145,7 +145,7 @@ int fss_ensemble_create(const fss_config* cfg, fss_ensemble** out) {
     }
     std::unique_ptr<fss_ensemble> e(new fss_ensemble());
     e->cfg = *cfg;
-    e->cfg.block_threads = kPersistentThreads;  // items hold at most one block of targets
+    e->cfg.block_threads = kPersistentThreads + 32;  // the persistent kernel's warps
     e->cfg.targets_per_thread = 1;
     e->cfg.src_parts = 1;
     e->cfg.autotune = 0;
@@ -180,6 +180,7 @@ int fss_ensemble_add(fss_ensemble* e, int64_t n, const double* state5, const dou
     fss_ctx* c = nullptr;
     int rc = fss_create(&e->cfg, &c);
     if (rc) return rc;
+    c->member = true;
     rc = fss_set_particles(c, n, state5, area);
     if (rc) {
         set_last_error(fss_last_error(c));
@@ -246,11 +247,14 @@ int fss_ensemble_build(fss_ensemble* e) {
                 const Segment& sg = L.segs[k];
                 w += (sg.kind == 0) ? double(ls[sg.b] - ls[sg.a]) : double(sg.b - sg.a);
             }
-            it.t0 = int32_t(it.t0 + po);
+            if (it.leaf < 0) it.t0 = int32_t(it.t0 + po);
             it.g0 += sbase;
             it.g1 += sbase;
             it.part = 0;
-            if (it.leaf >= 0) it.leaf += int32_t(lo);
+            if (it.leaf >= 0) {
+                w *= ls[it.leaf + 1] - ls[it.leaf];  // pairs
+                it.leaf += int32_t(lo);
+            }
             items.push_back(it);
             cost.push_back(w);
         }
@@ -279,7 +283,7 @@ int fss_ensemble_build(fss_ensemble* e) {
     }
     lstart.push_back(int32_t(e->ntot));
     e->max_leaf_level = maxTL - 1;
-    // longest source lists first across all members
+    // items of the most pairs first across all members
     {
         std::vector<size_t> order(items.size());
         for (size_t k = 0; k < order.size(); k++) order[k] = k;

@@ -170,6 +170,27 @@ int plane_parts(double blocks, double sources, int most) {
     return best;
 }
 
+// FP32 direct sum: targets per item, whose sources are one of P parts, at
+// target t0 of n.  An item's targets are summed on their own, so the choice
+// changes no result.  256 (a block's most) in whole rounds of the 740 blocks
+// that run at once, the rest in 128s and then 64s, so that the last round ends
+// evenly; fewer targets than a round in 128s, 64s or 32s.  Measured, us per
+// right-hand side: in 128s, 64s, 32s 700 particles 19.0 15.2 12.7; 2,001 19.5
+// 15.1 14.6; 5,000 24.2 22.4 27.7; with all in 256s, and the rest in 128s, in
+// 64s, in both: 10,001 60.0 54.2 53.5 54.1; 14,982 103.6 99.1 99.4
+// 99.5; 20,011 175.3 173.9 167.6 166.8; 32,000 409 405 397 395; 60,000 1396
+// 1368 1342 1338.
+int64_t direct_group(int64_t n, int64_t t0, int parts) {
+    auto items = [&](int64_t g) { return (n + g - 1) / g * parts; };
+    if (items(256) >= 740) {
+        const int64_t whole = n / 256 * parts / 740 * 740 / parts * 256;
+        return t0 < whole ? 256 : (t0 < (whole + n) / 2 ? 128 : 64);
+    }
+    if (items(128) >= 740) return 128;
+    if (items(64) >= 500) return 64;
+    return 32;
+}
+
 // Lists of the direct sum: blocks of targets x P chunks of the sources.
 int build_direct_lists(fss_ctx* c) {
     const int64_t n = c->n;
@@ -201,10 +222,13 @@ int build_direct_lists(fss_ctx* c) {
         c->shard_lo = t_lo * TB;
         c->shard_hi = std::min<int64_t>(n, t_hi * TB);
     }
-    for (int64_t t = t_lo; t < t_hi; t++) {
-        const int64_t t0 = t * TB, nt = std::min<int64_t>(TB, n - t0);
+    const int64_t t_first = t_lo * TB, t_end = std::min<int64_t>(n, t_hi * TB);
+    c->shape.max_targets = c->fp64 ? TB : int(direct_group(t_end - t_first, 0, P));
+    for (int64_t t0 = t_first, nt = 0; t0 < t_end; t0 += nt) {
+        nt = std::min<int64_t>(c->fp64 ? TB : direct_group(t_end - t_first, t0 - t_first, P), t_end - t0);
         for (int p = 0; p < P; p++) {
-            L.items.push_back(WorkItem{int32_t(t0), int32_t(nt), p, p + 1, p, -1});
+            L.items.push_back(WorkItem{int32_t(t0), int32_t(nt), p, p + 1, p, -1,
+                                       pair_split(double(L.segs[p].b - L.segs[p].a), int(nt), 4), 0});
             L.n_tiles += (L.segs[p].b - L.segs[p].a + c->shape.tile - 1) / c->shape.tile;
         }
     }
@@ -511,17 +535,46 @@ int build_tree(fss_ctx* c) {
     return FSS_OK;
 }
 
-// Block shape for the treecode's pair kernel: the configured one, or (FP32)
-// the smallest supported block whose consumer threads cover the largest leaf
-// (so that no leaf needs a second chunk).
+// Block shape for the treecode's pair kernel: the configured one, or the
+// smallest.
 PairShape choose_shape(fss_ctx* c) {
-    if (c->cfg.block_threads > 0) return pairs_shape(c->fp64, c->cfg.block_threads, c->cfg.targets_per_thread);
-    if (c->fp64) return pair_shapes(true).front();
-    int maxleaf = 1;
-    for (int64_t l = 0; l < c->nleaf; l++) maxleaf = std::max(maxleaf, c->leaf_start_h[l + 1] - c->leaf_start_h[l]);
-    for (const PairShape& sh : pair_shapes(c->fp64))
-        if (sh.per_thread == 1 && sh.targets() >= maxleaf) return sh;
-    return pair_shapes(c->fp64).back();
+    return pairs_shape(c->fp64, c->cfg.block_threads, c->cfg.targets_per_thread);
+}
+
+// FP32 engine: targets per item of a leaf whose lists are split into `parts`.
+// An item's targets are summed on their own, so the choice changes no result,
+// and it is the only way to give every SM work on a small problem, whose
+// source split is part of the result.  96 at a time unless that leaves the 740
+// blocks that run at once idle, then 64 (pairs of targets a lane), then 32.
+// Measured, us per right-hand side with whole leaves and with 96, 64, 32: 20
+// leaves of 128 particles 23.0 22.8 18.8 16.9; 20 of 200 31.2 22.9 19.9 16.9;
+// 80 of 128 37.3 36.7 31.6 31.1; 80 of 250 109 72.3 72.2 73.1; 320 of 218 251
+// 230 233 249; 1280 of 128 527 517 541 565; 5120 of 128 2473 2438 2533 2693;
+// 20 of 32 11.4 (whole) 12.5 (32).  With 1 to 4 rounds of blocks, some leaves
+// in 64s and 32s leave a finer tail (items start in the order of their pairs):
+// 1332 -> 1291 us per step of 100,003 particles.  Where target clusters'
+// launches fill the SMs as well, leaves of less than 192 stay whole and larger
+// ones are cut in 128s: per step 40,962 particles in leaves of 128 394 us (in 96s
+// and 128s 410); 20,011 in leaves of 250 286 us (whole 352).
+void leaf_group(const fss_ctx* c, int parts, ListInput& in) {
+    auto items = [&](int g) {
+        int64_t k = 0;
+        for (int64_t l = 0; l < c->nleaf; l++) {
+            const int nt = c->leaf_start_h[l + 1] - c->leaf_start_h[l];
+            k += nt == 0 ? 0 : leaf_items(nt, g);
+        }
+        return k * parts;
+    };
+    if (!c->tlists.empty()) {
+        in.group = 128;
+        return;
+    }
+    if (items(96) >= 740) {
+        in.group = 96;
+        in.mix = items(96) < 4 * 740;
+    } else {
+        in.group = (items(64) >= 500 || c->n < 64 * c->nleaf) ? 64 : 32;
+    }
 }
 
 // Work items, tiles and copies of the current lists for one block shape;
@@ -536,11 +589,11 @@ int materialize(fss_ctx* c, PairShape shape) {
     in.n = n;
     in.leaf_start = c->leaf_start_h.data();
     in.tile = shape.tile;
-    int P = c->cfg.src_parts;
+    int P = c->cfg.src_parts, maxleaf = 1;
+    for (int64_t l = 0; l < c->nleaf; l++) maxleaf = std::max(maxleaf, c->leaf_start_h[l + 1] - c->leaf_start_h[l]);
     if (P <= 0) {
         // blocks of targets: the smallest of these that holds the largest leaf
-        int maxleaf = 1, TB = 256;
-        for (int64_t l = 0; l < c->nleaf; l++) maxleaf = std::max(maxleaf, c->leaf_start_h[l + 1] - c->leaf_start_h[l]);
+        int TB = 256;
         for (int tb : {192, 160, 128})
             if (tb >= maxleaf) TB = tb;
         if (c->cfg.block_threads > 0) TB = shape.threads - 32;
@@ -551,6 +604,9 @@ int materialize(fss_ctx* c, PairShape shape) {
         if (c->fp64) P = plane_parts(c->list_blocks, c->list_sources, 16);
     }
     in.parts = P;
+    if (!c->fp64 && !c->member) leaf_group(c, P, in);
+    c->shape.max_targets = in.group > 0 ? std::min(maxleaf, in.group + in.group / 2) : maxleaf;
+    in.cluster_warps = cluster_shape(c->fp64, int64_t(c->tlists.size()) * P).warps();
     in.all_leaves = c->resort;
     c->parts = P;
     build_lists(in, c->alists, c->tlists, c->lists);
@@ -630,9 +686,7 @@ int materialize(fss_ctx* c, PairShape shape) {
     c->pstride = down ? n + L.n_proxy : n;
     CU(c->partials.ensure(sizeof(double4) * size_t(P + (down ? 1 : 0)) * size_t(c->pstride)));
     // the downward evaluation: a leaf and the clusters above it
-    c->max_leaf = 1;
-    for (int64_t l = 0; l < c->nleaf; l++)
-        c->max_leaf = std::max(c->max_leaf, c->leaf_start_h[l + 1] - c->leaf_start_h[l]);
+    c->max_leaf = maxleaf;
     c->max_coefs = 1;
     for (size_t i = 0; i < L.leaf_anc.size(); i += kMaxLevels) {
         int k = 0;
@@ -659,8 +713,8 @@ int launch_cluster_pairs(fss_ctx* c, cudaStream_t st, bool want_psi) {
     const ListOutput& L = c->lists;
     const int nl = int(L.n_leaf_items), nall = int(L.items.size());
     if (nall > nl)
-        CU(launch_pairs(st, c->fp64, want_psi, cluster_shape(c->fp64, L.max_cluster_k), nall - nl, c->src.p,
-                        c->segs.as<Segment>(), c->leaf_start.as<int32_t>(), c->items.as<WorkItem>() + nl,
+        CU(launch_pairs(st, c->fp64, want_psi, cluster_shape(c->fp64, int64_t(c->tlists.size()) * c->parts), nall - nl,
+                        c->src.p, c->segs.as<Segment>(), c->leaf_start.as<int32_t>(), c->items.as<WorkItem>() + nl,
                         c->partials.as<double4>(), c->pstride, c->err_flag.as<int>(), PairCtl{c->wait_ns, -1, 0}));
     return FSS_OK;
 }
@@ -1263,7 +1317,11 @@ double lane_pairs(const fss_ctx* c, int64_t i0, int64_t i1) {
             src += sg.kind == 0 ? double(c->leaf_start_h[sg.b] - c->leaf_start_h[sg.a]) : double(sg.b - sg.a);
         }
         const double quads = std::ceil(src / 4.0);
-        const int nt = it.leaf >= 0 ? c->leaf_start_h[it.leaf + 1] - c->leaf_start_h[it.leaf] : it.nt;
+        int nt = it.nt;
+        if (it.leaf >= 0) {
+            nt = std::max(0, c->leaf_start_h[it.leaf + 1] - c->leaf_start_h[it.leaf] - it.t0);
+            if (it.nt > 0) nt = std::min(nt, it.nt);
+        }
         sum += 32.0 * double(nt / 32) * 4.0 * quads;
         if (nt % 32) sum += 32.0 * 4.0 * std::ceil(quads / double(32 / (nt % 32)));
     }

@@ -30,15 +30,17 @@ struct Segment {
     int32_t pad;
 };
 
-// One block's work.  leaf >= 0: the targets are that leaf's current
-// particles, taken in chunks (chunk_targets); leaf < 0: the targets are
-// [t0, t0 + nt).  Sources: segments [g0, g1).  Results go to partial slot
+// One block's work.  leaf >= 0: the targets are that leaf's current particles
+// from the t0-th on, at most nt of them (nt = 0: all the rest); leaf < 0: the
+// targets are [t0, t0 + nt).  Sources: segments [g0, g1).  Results go to partial slot
 // `part`.
 struct WorkItem {
     int32_t t0, nt;
     int32_t g0, g1;
     int32_t part;
     int32_t leaf;
+    int32_t split;  // FP32: subsets of the targets that different warps sum
+    int32_t pad;
 };
 
 // Targets of a work item that one pass of a pair block serves: up to kMaxFull

@@ -38,15 +38,12 @@ struct EpiArgs {
     const int32_t* order = nullptr;
 };
 
-// Pair-kernel block.  FP32 (k_pairs.cu): one producer warp and consumer warps
-// with one target a thread.  FP64 (k_plane.cu): threads / 32 - 1 warps, which
-// share an item's sources.
+// Pair-kernel block: threads / 32 - 1 warps, which share an item's sources.
 struct PairShape {
     int threads = 160;
     int per_thread = 1;
     int tile = 256;
-    int depth = 4;  // ring slots (tiles in flight)
-    int targets() const { return (threads - 32) * per_thread; }
+    int max_targets = 256;  // of most items (FP32: how many the block has room for)
     int warps() const { return threads / 32 - 1; }
 };
 
@@ -95,9 +92,8 @@ void launch_gather(cudaStream_t st, bool fp64, int64_t n, const double* in5, con
 const std::vector<PairShape>& pair_shapes(bool fp64);
 // The supported shape with `threads`, or the default (160).
 PairShape pairs_shape(bool fp64, int threads, int per_thread);
-// Block for work items of k targets (target clusters: their interpolation
-// points): the smallest of 64, 96, 128, 160 threads whose consumers hold them.
-PairShape cluster_shape(bool fp64, int k);
+// Block for `items` target clusters (times source parts).
+PairShape cluster_shape(bool fp64, int64_t items);
 cudaError_t launch_pairs(cudaStream_t st, bool fp64, bool psi, PairShape shape, int nitems, const void* src,
                          const Segment* segs, const int32_t* leaf_start, const WorkItem* items, double4* partials,
                          int64_t pstride, int* err, PairCtl ctl);
@@ -105,7 +101,7 @@ cudaError_t launch_pairs(cudaStream_t st, bool fp64, bool psi, PairShape shape, 
 cudaError_t launch_plane_pairs(cudaStream_t st, bool psi, int warps, int nitems, const void* src, const Segment* segs,
                                const int32_t* leaf_start, const WorkItem* items, double4* partials, int64_t pstride,
                                int* err, PairCtl ctl);
-constexpr int kPersistentThreads = 160;
+constexpr int kPersistentThreads = 128;
 cudaError_t launch_pairs_persistent(cudaStream_t st, int nitems, const void* src, const Segment* segs,
                                     const int32_t* leaf_start, const WorkItem* items, int* queue, double4* partials,
                                     int64_t pstride, int* err, int blocks, PairCtl ctl);

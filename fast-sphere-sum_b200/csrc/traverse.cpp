@@ -290,6 +290,9 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
             }
         }
         const int chunks = std::max(1, chunk_count(nt_est));
+        // a leaf's targets in items of in.group, the last of them open-ended
+        const int grp = !in.mix || leaf % 16 > 1 ? in.group : (leaf % 16 == 0 ? 32 : 64);
+        const int subs = leaf >= 0 ? leaf_items(nt_est, grp) : 1;
         for (int p = 0; p < P; p++) {
             const int32_t base = int32_t(out.segs.size());
             double w = 0;
@@ -313,10 +316,15 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
                     out.segs.push_back(e);
                 w += est[k];
             }
-            out.n_tiles += int64_t(chunks) * (int64_t(w + in.tile - 1) / in.tile);
-            // a block's run time follows its source count (its warps run
-            // side by side), so the longest source lists go first
-            items.push_back({w * chunks, WorkItem{t0, nt_item, base, int32_t(out.segs.size()), p, leaf}});
+            out.n_tiles += int64_t(std::max(chunks, subs)) * (int64_t(w + in.tile - 1) / in.tile);
+            // a block's run time follows its pairs, so the most go first
+            const int32_t g1 = int32_t(out.segs.size());
+            for (int s = 0; s < subs; s++) {
+                const bool last = s + 1 == subs;
+                const int32_t first = s * grp, nt = last ? nt_est - first : grp;
+                items.push_back({w * nt, WorkItem{t0 + first, last ? nt_item : grp, base, g1, p, leaf,
+                                                  pair_split(w, nt, leaf >= 0 ? 4 : in.cluster_warps), 0}});
+            }
         }
     };
     auto flush_items = [&]() {
@@ -369,6 +377,41 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
             }
         }
     }
+}
+
+// ---------------------------------------------------------------- FP32 items
+
+int pair_split(double sources, int targets, int warps) {
+    // a warp's time on a tile: 1 for 32 targets, 1.76 for 64 (two a lane), the
+    // share of the lanes that r targets left over occupy, and a fixed part
+    // for each
+    const int tile = tile_capacity(false), chunk = std::min(targets, 256);  // a pass of the kernel
+    const int full = chunk / 32, r = chunk % 32, G = full + (r > 0);
+    const double tiles = std::max(sources, 1.0) / tile;
+    const int whole = int(tiles);
+    int best = 1;
+    double best_t = 1e300;
+    for (int H : {1, 2, 4}) {
+        if (warps % H) continue;
+        const int stride = warps / H;
+        double busiest = 0, slowest = 0;
+        for (int j = 0; j < stride; j++) {
+            double load = (whole - j + stride - 1) / stride;
+            if (whole % stride == j) load += tiles - whole;
+            busiest = std::max(busiest, load);
+        }
+        for (int h = 0; h < H; h++) {
+            const int ga = G * h / H, gb = G * (h + 1) / H, f = std::min(gb, full) - ga;
+            const double t = 1.76 * (f / 2) + (f % 2) + (gb > full ? 0.1 + 1.0 / (32 / r) : 0.0);
+            slowest = std::max(slowest, t);
+        }
+        const double t = busiest * (slowest + 0.1);
+        if (t < 0.99 * best_t) {
+            best_t = t;
+            best = H;
+        }
+    }
+    return best;
 }
 
 // ---------------------------------------------------------------- sharding

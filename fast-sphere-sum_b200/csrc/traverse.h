@@ -1,5 +1,6 @@
 // traverse.h -- interaction lists of the icosahedral treecode (host).
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -59,7 +60,21 @@ struct ListInput {
     int tile = 256;                     // sources per shared-memory tile
     int parts = 1;                      // source-list split
     bool all_leaves = false;            // items also for leaves empty at the build
+    int cluster_warps = 4;              // of the block that takes a target cluster
+    int group = 0;                      // targets per item of a leaf (a multiple of 32; 0: the whole leaf)
+    bool mix = false;                   // of 16 leaves, one in items of 32 and one of 64 all the same
 };
+
+// Items of a leaf of nt particles in groups of `group` (0: one): as many as
+// nt / group rounds to, so that none is left with a few targets.
+inline int leaf_items(int nt, int group) { return group > 0 ? std::max(1, (nt + group / 2) / group) : 1; }
+
+// FP32 engine: in how many subsets (1, 2 or 4) the warps of a block take an
+// item's targets.  One has every warp sum whole tiles of sources for all
+// targets, which needs a multiple of their number of tiles to keep them
+// equally busy; with more, the warps share the targets as well.  The subsets
+// change no result.
+int pair_split(double sources, int targets, int warps);
 
 struct ListOutput {
     std::vector<Segment> segs;      // per work item, in list order

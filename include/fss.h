@@ -96,10 +96,8 @@ typedef struct fss_config {
     int32_t use_graph;     /* capture the RK4 step in a CUDA graph */
     int32_t src_parts;     /* split each target's source list in this many parts
                               (0 = automatic) */
-    int32_t block_threads; /* threads per interaction block: one producer warp
-                              plus one consumer thread per target, 160, 192,
-                              224 or 288 (0 = automatic: the smallest block
-                              whose consumers hold the largest leaf) */
+    int32_t block_threads; /* shape of an interaction block: 160, 192, 224 or
+                              288 for 4, 5, 6 or 8 warps (0 = automatic: 4) */
     int32_t targets_per_thread; /* 1 */
     int32_t autotune;      /* at fss_set_particles: 1 = time every supported
                               block shape of the pair kernel on the actual
