@@ -482,7 +482,7 @@ def kernel_rooflines(prof, steps, n, up_bytes, peaks):
 
     up_ms = sum(prof[k][0] for k in ("upward_leaf", "upward_combine") if k in prof) / (4 * steps)
     if up_ms > 0:
-        add("upward pass (k_up_leaf, k_up_sums, k_up_proxies)", up_ms, float(up_bytes), "RHS")
+        add("upward pass (k_up_leaf, k_up_proxies)", up_ms, float(up_bytes), "RHS")
     if "resort" in prof:
         add("tree build: per-step re-sort (k_part_keys, k_part_scan, k_part_bucket, k_part_place, "
             "k_resort_commit)", prof["resort"][0] / steps, float(n) * (24 + 8 + 16), "step")
