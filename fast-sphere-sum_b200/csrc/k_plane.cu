@@ -31,6 +31,11 @@
 // target.  The map keeps the relative precision of x - c near the targets, so
 // neighbours' differences carry the rounding of the positions and no more.
 //
+// The map holds on the unit sphere alone.  Sources or targets that are not on
+// it (kOnSphere) are summed in space, at 14 operations a pair: a warp's share
+// of a tile that has such a source, and every share for a chunk of targets
+// that has such a target.
+//
 // Bound by the FP64 pipe, 80% busy (20 of the 27 cycles that a pair takes a
 // warp).  Per right-hand side, before and now: treecode of 163,842 particles
 // (n = 8, theta = 0.7; 1.29e9 lane pairs) 1.347 and 0.918 ms; direct sum of
@@ -58,9 +63,20 @@ constexpr double kSelfR2 = 1e-200;
 // they add nothing.
 constexpr double kFarAway = 1e100;
 
+// | |x|^2 - 1 | of a point on the unit sphere: the rounding of a normalised
+// position is below 2^-50.
+constexpr double kOnSphere = 0x1p-48;
+__device__ __forceinline__ double norm2(double x, double y, double z) {
+    return __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x)));
+}
+__device__ __forceinline__ bool on_sphere(double x, double y, double z) {
+    return fabs(norm2(x, y, z) - 1.0) <= kOnSphere;  // false for a non-finite position
+}
+
 // The plane of a pass, in shared memory.
 struct PlaneShared {
     double c[3], e1[3], e2[3];
+    int flat;     // the chunk's targets are all on the sphere
     int next[2];  // lowest target left to a later pass (alternating)
 };
 struct Plane {
@@ -84,7 +100,7 @@ struct Plane {
 // Explicitly rounded operations: a target and the same point as a source must
 // map to the same bits.
 __device__ __forceinline__ void plane_map(const Plane& p, double x, double y, double z, double& u, double& v) {
-    const double nn = __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x)));
+    const double nn = norm2(x, y, z);
     double n = __fma_rn(-0.5, nn, 1.5);
     n = __dmul_rn(n, __fma_rn(__dmul_rn(-0.5, nn), __dmul_rn(n, n), 1.5));
     x = __dmul_rn(x, n);
@@ -136,6 +152,10 @@ __device__ __forceinline__ void plane_around(double x, double y, double z, Plane
 // A lane's accumulators, one slot per target.
 struct alignas(16) Acc {
     double u, v;
+};
+// The same for the sources summed in space: their share of A.
+struct Acc3 {
+    double x, y, z;
 };
 
 // log2 of r2 (positive, finite) beside its reciprocal's approximation y: y
@@ -237,29 +257,93 @@ __device__ __forceinline__ void plane_fold(const double* __restrict__ share, int
     }
 }
 
+// Pairs of NT targets t of a lane with sources j0, j0 + step, ... < n as they
+// landed, in space: A = sum w_j d / |d|^2, d = x_j - x_i, exact for neighbours,
+// at any radius.  A source at the target's position adds nothing: r^2 starts
+// from kSelfR2, so that its reciprocal is finite and multiplies d = 0.
+template <bool PSI, int NT>
+__device__ __forceinline__ void space_pairs(const double4* __restrict__ s, int j0, int n, int step,
+                                            const double4 (&t)[NT], Acc3 (&a)[NT], double (&ap)[NT],
+                                            const double* __restrict__ lg) {
+#pragma unroll
+    for (int k = 0; k < NT; k++) {
+        a[k] = Acc3{};
+        ap[k] = 0.0;
+    }
+#pragma unroll(PSI ? 1 : 2)
+    for (int j = j0; j < n; j += step) {
+        const double4 q = s[j];
+#pragma unroll
+        for (int k = 0; k < NT; k++) {
+            const double dx = q.x - t[k].x, dy = q.y - t[k].y, dz = q.z - t[k].z;
+            const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, kSelfR2)));
+            const double sc = q.w * rcp_fast(r2);
+            a[k].x = fma(sc, dx, a[k].x);
+            a[k].y = fma(sc, dy, a[k].y);
+            a[k].z = fma(sc, dz, a[k].z);
+            if (PSI) {
+                const double l = log2_beside(r2, rcp_seed(r2), lg);
+                ap[k] = fma(q.w, (r2 > kSelfR2) ? l : 0.0, ap[k]);
+            }
+        }
+    }
+}
+
+// A warp's share of a tile for its lanes' NT targets (tgt[32 k]) in space,
+// added to the lane's accumulators.
+template <bool PSI, int NT>
+__device__ __forceinline__ void space_fold(const double4* __restrict__ share, int j0, int n, int step,
+                                           const double4* __restrict__ tgt, Acc3* acc, double* accp,
+                                           const double* lg) {
+    const int lane = threadIdx.x & 31;
+    double4 t[NT];
+    Acc3 a[NT];
+    double ap[NT];
+#pragma unroll
+    for (int k = 0; k < NT; k++) t[k] = tgt[32 * k];
+    space_pairs<PSI, NT>(share, j0, n, step, t, a, ap, lg);
+#pragma unroll
+    for (int k = 0; k < NT; k++) {
+        Acc3& o = acc[32 * k + lane];
+        o.x += a[k].x;
+        o.y += a[k].y;
+        o.z += a[k].z;
+        if (PSI) accp[32 * k + lane] += ap[k];
+    }
+}
+
 // A warp's share of a landed tile -- n sources from `in` -- mapped to the
 // plane (lane L takes sources L, L + 32, ...: conflict-free) into the warp's
 // own arrays u, v, w of SHARE entries, padded to whole units with w = 0; the
-// lane's sums of w and w log2(1 + rho) added to wsum and lsum.
+// lane's sums of w and w log2(1 + rho) added to wsum and lsum.  False when a
+// source is not on the sphere: the share is to be summed in space (and
+// nothing is added).
 template <bool PSI, int SHARE>
-__device__ __forceinline__ void map_share(const double4* __restrict__ in, double* __restrict__ out, int n,
+__device__ __forceinline__ bool map_share(const double4* __restrict__ in, double* __restrict__ out, int n,
                                           const Plane& p, double& wsum, double& lsum) {
     const int lane = threadIdx.x & 31;
     const int padded = (n + 1) & ~1;
+    double ws = 0, ls = 0;
+    bool flat = true;
 #pragma unroll 2
     for (int j = lane; j < padded; j += 32) {
         double u = kFarAway, v = 0, w = 0;
         if (j < n) {
             const double4 q = in[j];
+            flat = flat && on_sphere(q.x, q.y, q.z);
             plane_map(p, q.x, q.y, q.z, u, v);
             w = q.w;
         }
         out[j] = u;
         out[SHARE + j] = v;
         out[2 * SHARE + j] = w;
-        wsum += w;
-        if (PSI) lsum += w * lg2_fast(fma(v, v, fma(u, u, 1.0)));
+        ws += w;
+        if (PSI) ls += w * lg2_fast(fma(v, v, fma(u, u, 1.0)));
     }
+    if (!__all_sync(0xffffffffu, flat)) return false;
+    wsum += ws;
+    if (PSI) lsum += ls;
+    return true;
 }
 
 // Tile header written by warp 0 before the slot's arrive (every warp reads it
@@ -302,6 +386,7 @@ struct PairSmem {
     double4 ring[kDepth * kTile];
     double mapped[WARPS * 3 * kShare];
     Acc acc[WARPS * kSlots];
+    Acc3 acc3[WARPS * kSlots];
     double2 tpos[kSlots];
     double wz[WARPS * kSlots];
     double accp[PSI ? WARPS * kSlots : 1];
@@ -317,7 +402,8 @@ struct PairBars {
 // One work item: every chunk of targets against every tile of its segments.
 // Warp 0 packs and issues the tiles, one ahead of the one in use.  Every warp
 // maps its share of a landed tile to the plane, releases the slot through
-// empty, and takes its share for all targets of the chunk: cn >> 5 targets a
+// empty (a share summed in space is read from the slot, which is released
+// after), and takes its share for all targets of the chunk: cn >> 5 targets a
 // lane (a source loaded serves them all) and, for the r = cn & 31 left over,
 // L = 32 / r lanes a target, which split the share between them.  So the
 // warps' work is equal whatever the count of targets (one warp per 32 targets
@@ -405,14 +491,19 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             }
             const double d = mx * fx + my * fy + mz * fz, mm = mx * mx + my * my + mz * mz;
             const bool mean = d > 0.0 && d * d > 2.0 * kMinCos * kMinCos * mm;
-            if (lane == 0) plane_around(mean ? mx : fx, mean ? my : fy, mean ? mz : fz, *ps);
+            if (lane == 0) {
+                plane_around(mean ? mx : fx, mean ? my : fy, mean ? mz : fz, *ps);
+                ps->flat = 1;
+            }
         }
         Acc* acc = sm.acc + warp * kSlots;
+        Acc3* acc3 = sm.acc3 + warp * kSlots;
         double* accp = PSI ? sm.accp + warp * kSlots : sm.accp;
         double* wz = sm.wz + warp * kSlots;
         double* mapped = sm.mapped + warp * 3 * SHARE;
         for (int k = lane; k < 32 * (full + 1); k += 32) {
             acc[k] = Acc{};
+            acc3[k] = Acc3{};
             wz[k] = 0;
             if (PSI) accp[k] = 0.0;
         }
@@ -425,9 +516,11 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                 double2 p;
                 plane_map(plane, v.x, v.y, v.z, p.x, p.y);
                 sm.tpos[i] = p;
+                if (!on_sphere(v.x, v.y, v.z)) ps->flat = 0;
             }
         }
         __syncthreads();
+        const bool flat = ps->flat != 0;
         double wsum = 0, lsum = 0;
         while (!rs.failed) {
             if (warp == 0 && !packed) {
@@ -443,17 +536,32 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             const SlotHdr h = br.hdr[slot];
             const int nu = (h.count + UNIT - 1) / UNIT;
             const int q0 = nu * warp / WARPS, q1 = nu * (warp + 1) / WARPS, nq = q1 - q0;
-            if (nq > 0) {
+            const double4* share = sm.ring + slot * kTile + q0 * UNIT;
+            const int ns = min(h.count, q1 * UNIT) - q0 * UNIT;
+            bool space = nq > 0 && !flat;
+            if (nq > 0 && flat) {
                 Plane plane;
                 plane.load(*ps);
-                map_share<PSI, SHARE>(sm.ring + slot * kTile + q0 * UNIT, mapped,
-                                         min(h.count, q1 * UNIT) - q0 * UNIT, plane, wsum, lsum);
+                space = !map_share<PSI, SHARE>(share, mapped, ns, plane, wsum, lsum);
+            }
+            if (space) {
+                const double4* tgt = src + t0 + c0;
+                int g = 0;
+                for (; g + 2 <= full; g += 2)
+                    space_fold<PSI, 2>(share, 0, ns, 1, tgt + 32 * g + lane, acc3 + 32 * g,
+                                       PSI ? accp + 32 * g : accp, sm.lg);
+                if (g < full)
+                    space_fold<PSI, 1>(share, 0, ns, 1, tgt + 32 * g + lane, acc3 + 32 * g,
+                                       PSI ? accp + 32 * g : accp, sm.lg);
+                if (r > 0)
+                    space_fold<PSI, 1>(share, lane % L, ns, L, tgt + 32 * full + min(lane / L, r - 1),
+                                       acc3 + 32 * full, PSI ? accp + 32 * full : accp, sm.lg);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&br.empty[slot]);
             rs.taken++;
             if (h.count == 0) break;
-            if (nq > 0) {
+            if (nq > 0 && !space) {
                 const bool gd = h.guard != 0;
                 const auto* tp = sm.tpos + lane;
                 switch (full) {
@@ -496,7 +604,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             if ((done >> j) & 1) continue;
             const double4 v = src[t0 + c0 + tgt];
             const double x = v.x, y = v.y, z = v.z;
-            if (tgt != first && x * ps->c[0] + y * ps->c[1] + z * ps->c[2] <= kMinCos) {
+            if (flat && tgt != first && x * ps->c[0] + y * ps->c[1] + z * ps->c[2] <= kMinCos) {
                 atomicMin(&ps->next[rs.pass & 1], tgt);
                 continue;
             }
@@ -504,6 +612,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             const bool rest = tgt >= 32 * full;
             const int s0 = rest ? 32 * full + L * (tgt - 32 * full) : tgt, ns = rest ? L : 1;
             double bu = 0, bv = 0, bp = 0, bz = 0, wtot = 0, ltot = 0;
+            Acc3 in_space{};
             for (int w = 0; w < WARPS; w++) {
                 wtot += sm.wsum[w];
                 ltot += sm.lsum[w];
@@ -511,13 +620,23 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                     const Acc& a = sm.acc[w * kSlots + k];
                     bu += a.u;
                     bv += a.v;
+                    const Acc3& a3 = sm.acc3[w * kSlots + k];
+                    in_space.x += a3.x;
+                    in_space.y += a3.y;
+                    in_space.z += a3.z;
                     bz += sm.wz[w * kSlots + k];
                     if (PSI) bp += sm.accp[w * kSlots + k];
                 }
             }
-            const double2 p = sm.tpos[tgt];
-            partials[int64_t(it.part) * pstride + t0 + c0 + tgt] =
-                target_sum<PSI>(*ps, wtot, ltot, x, y, z, p.x, p.y, bu, bv, bp, bz);
+            double4 o = make_double4(0.0, 0.0, 0.0, bp);
+            if (flat) {
+                const double2 p = sm.tpos[tgt];
+                o = target_sum<PSI>(*ps, wtot, ltot, x, y, z, p.x, p.y, bu, bv, bp, bz);
+            }
+            o.x += in_space.x;
+            o.y += in_space.y;
+            o.z += in_space.z;
+            partials[int64_t(it.part) * pstride + t0 + c0 + tgt] = o;
         }
         __syncthreads();
         // the next pass: around the first target left, else the next chunk.

@@ -17,7 +17,10 @@
  * particle {x, y, z, zeta (relative vorticity), tracer}; area is one double
  * per particle; modify has the same layout as the state and is fully
  * overwritten with {u_x, u_y, u_z, dzeta/dt = -2 omega u_z, 0}.  Time is in
- * days, the sphere has radius 1, omega = 2 pi.
+ * days, the sphere has radius 1, omega = 2 pi.  A particle off the sphere is
+ * summed where it is, in either precision: pairs contribute
+ * -(1/2pi) w_j x_i x (x_j - x_i) / |x_j - x_i|^2 to the velocity and
+ * -(1/4pi) w_j log(|x_j - x_i|^2 / 2) to the stream function.
  *
  * Every entry point returns an fss_status (0 = success); no exception
  * crosses this boundary.  A context is not thread-safe: one host thread at a

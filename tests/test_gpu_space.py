@@ -1,0 +1,84 @@
+"""The FP64 sums where the plane does not serve: they must come out as sums in
+space, target by target.
+
+Bound.  A term's differences, square, reciprocal and products are 16 roundings
+at most, on either side of the comparison in FP64; n terms are added in some
+order (n roundings of the partial sums); the cross product and the sums' last
+steps add 16 more: an error of at most (n + 32) u times the sum of the terms'
+magnitudes, u = 2^-53, and the reference, summed in extended precision, adds
+nothing to it.  A logarithm's terms are taken with 30 added to their magnitude:
+the parts that it is put together from (log2 of distances in the plane and of
+1 + rho, at most 2 + 2 log2(4 n) here) are larger than itself.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def points(n, seed):
+    rng = np.random.default_rng(seed)
+    s = np.zeros((n, 5))
+    s[:, :3] = rng.standard_normal((n, 3))
+    s[:, :3] /= np.linalg.norm(s[:, :3], axis=1, keepdims=True)
+    s[:, 3] = rng.standard_normal(n) * 5
+    return s, np.full(n, 4 * np.pi / n)
+
+
+def in_space(s, a):
+    """u, psi in extended precision, and the sums of the magnitudes of their terms."""
+    x = s[:, :3].astype(np.longdouble)
+    w = (s[:, 3] * a).astype(np.longdouble)
+    u, psi, mu, mp = np.empty(x.shape), np.empty(len(x)), np.empty(len(x)), np.empty(len(x))
+    for i in range(len(x)):
+        d = x - x[i]
+        r2 = (d * d).sum(1)
+        other = r2 > 0
+        r2 = np.where(other, r2, 1)
+        f = np.where(other, w / r2, 0)
+        lg = np.where(other, np.log(r2 / 2), 0)
+        u[i] = -np.cross(x[i], f @ d) / (2 * np.pi)
+        psi[i] = -(w @ lg) / (4 * np.pi)
+        radius = np.sqrt((x[i] ** 2).sum())
+        mu[i] = radius * (np.abs(f) * np.sqrt(r2)).sum() / (2 * np.pi)
+        mp[i] = np.abs(w) @ (np.abs(lg) + 30) / (4 * np.pi)
+    return u, psi, mu, mp
+
+
+def check(fss, s, a, method, levels, built=None):
+    u, psi, mu, mp = in_space(s, a)
+    with fss.Context(method=method, precision=fss.PREC_FP64, tree_levels=levels, theta=1e-3) as c:
+        c.set_particles(s if built is None else built, a)
+        out, p = c.rhs(s, a, psi=True)
+        alone = c.rhs(s, a)
+    eps = (len(s) + 32) * 2.0 ** -53
+    assert np.all(np.linalg.norm(out[:, :3] - u, axis=1) <= eps * mu)
+    assert np.all(np.linalg.norm(alone[:, :3] - u, axis=1) <= eps * mu)
+    assert np.all(np.abs(p - psi) <= eps * mp)
+
+
+ALL_PAIRS = [(0, 0), (1, 1), (1, 2)]  # direct sum; trees that resolve every pair
+
+
+@pytest.mark.parametrize("method,levels", ALL_PAIRS)
+@pytest.mark.parametrize("radius", [0.5, 1.0, 1 + 1e-9, 1.01, 1.5, 2.0])
+def test_any_radius(fss, radius, method, levels):
+    s, a = points(701, 3)
+    s[:, :3] *= radius
+    check(fss, s, a, method, levels)
+
+
+@pytest.mark.parametrize("method,levels", ALL_PAIRS)
+@pytest.mark.parametrize("digits", [4, 6, 10, 14])
+def test_rounded_positions(fss, digits, method, levels):
+    s, a = points(660, 5)
+    s[:, :3] = np.round(s[:, :3], digits)
+    check(fss, s, a, method, levels)
+
+
+@pytest.mark.parametrize("method,levels", ALL_PAIRS)
+def test_a_few_off_the_sphere(fss, method, levels):
+    """Sources and targets off the sphere among others on it."""
+    s, a = points(900, 7)
+    s[[3, 120, 121, 500, 899], :3] *= np.array([0.9, 1.1, 1 + 1e-12, 1.3, 1 - 1e-5])[:, None]
+    check(fss, s, a, method, levels)
