@@ -27,14 +27,16 @@
 //
 // so that a pair costs 10 FP64 operations (2 differences, 2 for r^2, 4 for
 // w / r^2, 2 accumulations) where differences in space cost 14; everything
-// else is done once per source and pass (about 40 operations) or once per
+// else is done once per source and chunk (about 40 operations) or once per
 // target.  The map keeps the relative precision of x - c near the targets, so
 // neighbours' differences carry the rounding of the positions and no more.
 //
-// The map holds on the unit sphere alone.  Sources or targets that are not on
-// it (kOnSphere) are summed in space, at 14 operations a pair: a warp's share
-// of a tile that has such a source, and every share for a chunk of targets
-// that has such a target.
+// The map holds on the unit sphere alone and serves targets on c's side of it
+// (kMinCos).  What it does not serve is summed in space, at 14 operations a
+// pair: a warp's share of a tile with a source off the sphere (kOnSphere), and
+// every share for a chunk with a target off it or with targets all over it
+// (a tree evaluated at other positions than its own: 163,842 particles 1.40 ms,
+// where a pass over the sources around each group of targets took 4.31).
 //
 // Bound by the FP64 pipe, 80% busy (20 of the 27 cycles that a pair takes a
 // warp).  Per right-hand side, before and now: treecode of 163,842 particles
@@ -51,8 +53,7 @@ namespace fss {
 constexpr int kUnroll = 2;       // units per step of the pair loop
 constexpr int kDepth = 2;        // ring depth (tiles in flight)
 constexpr int kTile = tile_capacity(true);
-constexpr double kMinCos = 0.2;  // a pass takes the targets with x.c above this
-constexpr int kNoTarget = 0x7fffffff;
+constexpr double kMinCos = 0.2;  // the plane serves targets with x.c above this
 constexpr int kSlots = 32 * (kMaxFull + 1);  // accumulator slots of a warp
 
 // What the guarded pair loop adds to r^2, so that a source at the target's
@@ -73,11 +74,10 @@ __device__ __forceinline__ bool on_sphere(double x, double y, double z) {
     return fabs(norm2(x, y, z) - 1.0) <= kOnSphere;  // false for a non-finite position
 }
 
-// The plane of a pass, in shared memory.
+// The plane of a chunk of targets, in shared memory.
 struct PlaneShared {
     double c[3], e1[3], e2[3];
-    int flat;     // the chunk's targets are all on the sphere
-    int next[2];  // lowest target left to a later pass (alternating)
+    int flat;  // it serves them
 };
 struct Plane {
     double c[3], a[3], b[3];
@@ -88,6 +88,9 @@ struct Plane {
             a[k] = s.e1[k];
             b[k] = s.e2[k];
         }
+    }
+    __device__ __forceinline__ bool serves(double x, double y, double z) const {
+        return x * c[0] + y * c[1] + z * c[2] > kMinCos;
     }
 };
 
@@ -126,10 +129,9 @@ __device__ __forceinline__ void plane_map(const Plane& p, double x, double y, do
     v = __dmul_rn(b, k);
 }
 
-// The plane around a target: c its direction, e1 and e2 by the branchless
+// The plane around (x, y, z): c its direction, e1 and e2 by the branchless
 // construction of Duff et al., "Building an orthonormal basis, revisited"
-// (JCGT 6, 2017).  A zero or non-finite position takes the pole (its own
-// sums are then whatever they are; the others' are not touched).
+// (JCGT 6, 2017).  Without a direction it is the pole.
 __device__ __forceinline__ void plane_around(double x, double y, double z, PlaneShared& s) {
     const double nn = x * x + y * y + z * z;
     const double r = rsqrt(nn);
@@ -353,8 +355,7 @@ struct SlotHdr {
 };
 
 struct RingState {
-    int issued, taken;  // tiles, over all passes
-    int pass;  // passes so far (selects PlaneShared::next)
+    int issued, taken;  // tiles, over all chunks
     bool failed;
 };
 
@@ -409,11 +410,7 @@ struct PairBars {
 // warps' work is equal whatever the count of targets (one warp per 32 targets
 // left the SM's quarters unequally loaded: leaves of 78 particles ran at 62%
 // of the rate of leaves of 128), and no warp waits for another's mapping.
-// The warps' sums are added at the end of the pass.  A pass over the sources
-// serves the chunk's targets on the side of the sphere of its plane's c: all
-// of them when the chunk is a leaf, a cluster or neighbours in space; targets
-// spread over the sphere are left to further passes, each around the first
-// one left.
+// The warps' sums are added at the end of the chunk.
 template <int WARPS, bool PSI>
 __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __restrict__ src,
                                          const Segment* __restrict__ segs, const int32_t* __restrict__ leaf_start,
@@ -430,12 +427,11 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
         nt = leaf_start[it.leaf + 1] - t0;
     }
     const int chunk = chunk_targets(nt);
-    uint32_t done = 0;  // bit j: target tid + 32 WARPS j of the chunk
-    for (int c0 = 0, first = 0; c0 < nt;) {
+    for (int c0 = 0; c0 < nt; c0 += chunk) {
         const int cn = min(chunk, nt - c0);
         const int full = cn >> 5, r = cn & 31;
         const int L = r > 0 ? 32 / r : 1;
-        // warp 0: the next tile into its slot (an empty one ends the pass),
+        // warp 0: the next tile into its slot (an empty one ends the chunk),
         // once every warp has mapped the tile before it there
         Window win;
         bool packed = false;  // the empty tile has been issued
@@ -470,29 +466,22 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             window_start(segs, leaf_start, it.g0, it.g1, win);
             issue();
         } else if (warp == 1) {
-            // c: the direction of the chunk's targets' mean on its first pass,
-            // when that serves the first of them; else the first one left
+            // c: the direction of the chunk's targets' mean
             double mx = 0, my = 0, mz = 0;
-            const double4 f = src[t0 + c0 + first];
-            const double fx = f.x, fy = f.y, fz = f.z;
-            if (first == 0) {
-                for (int i = lane; i < cn; i += 32) {
-                    const double4 v = src[t0 + c0 + i];
-                    mx += v.x;
-                    my += v.y;
-                    mz += v.z;
-                }
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    mx += __shfl_xor_sync(0xffffffffu, mx, off);
-                    my += __shfl_xor_sync(0xffffffffu, my, off);
-                    mz += __shfl_xor_sync(0xffffffffu, mz, off);
-                }
+            for (int i = lane; i < cn; i += 32) {
+                const double4 v = src[t0 + c0 + i];
+                mx += v.x;
+                my += v.y;
+                mz += v.z;
             }
-            const double d = mx * fx + my * fy + mz * fz, mm = mx * mx + my * my + mz * mz;
-            const bool mean = d > 0.0 && d * d > 2.0 * kMinCos * kMinCos * mm;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                mx += __shfl_xor_sync(0xffffffffu, mx, off);
+                my += __shfl_xor_sync(0xffffffffu, my, off);
+                mz += __shfl_xor_sync(0xffffffffu, mz, off);
+            }
             if (lane == 0) {
-                plane_around(mean ? mx : fx, mean ? my : fy, mean ? mz : fz, *ps);
+                plane_around(mx, my, mz, *ps);
                 ps->flat = 1;
             }
         }
@@ -516,7 +505,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                 double2 p;
                 plane_map(plane, v.x, v.y, v.z, p.x, p.y);
                 sm.tpos[i] = p;
-                if (!on_sphere(v.x, v.y, v.z)) ps->flat = 0;
+                if (!on_sphere(v.x, v.y, v.z) || !plane.serves(v.x, v.y, v.z)) ps->flat = 0;
             }
         }
         __syncthreads();
@@ -587,7 +576,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             sm.lsum[warp] = lsum;
         }
         if (warp > 0) rs.issued = rs.taken;
-        // every tile issued for this pass has been taken, so the counters
+        // every tile issued for this chunk has been taken, so the counters
         // agree in every warp unless a wait gave up
         rs.failed = __syncthreads_or(rs.failed) != 0;
         if (rs.failed) {
@@ -599,16 +588,10 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                     mbar_wait_bounded(&br.full[t % kDepth], uint32_t(t / kDepth) & 1, ctl.wait_ns);
             return;
         }
-        // the targets of this pass: their sums over the warps (and lanes)
-        for (int tgt = tid, j = 0; tgt < cn; tgt += 32 * WARPS, j++) {
-            if ((done >> j) & 1) continue;
+        // the targets' sums over the warps (and lanes)
+        for (int tgt = tid; tgt < cn; tgt += 32 * WARPS) {
             const double4 v = src[t0 + c0 + tgt];
             const double x = v.x, y = v.y, z = v.z;
-            if (flat && tgt != first && x * ps->c[0] + y * ps->c[1] + z * ps->c[2] <= kMinCos) {
-                atomicMin(&ps->next[rs.pass & 1], tgt);
-                continue;
-            }
-            done |= 1u << j;
             const bool rest = tgt >= 32 * full;
             const int s0 = rest ? 32 * full + L * (tgt - 32 * full) : tgt, ns = rest ? L : 1;
             double bu = 0, bv = 0, bp = 0, bz = 0, wtot = 0, ltot = 0;
@@ -639,17 +622,6 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             partials[int64_t(it.part) * pstride + t0 + c0 + tgt] = o;
         }
         __syncthreads();
-        // the next pass: around the first target left, else the next chunk.
-        // The other slot of `next` was last read before this barrier and is
-        // next used after the next pass's first barrier.
-        first = ps->next[rs.pass & 1];
-        rs.pass++;
-        if (tid == 0) ps->next[rs.pass & 1] = kNoTarget;
-        if (first == kNoTarget) {
-            c0 += chunk;
-            first = 0;
-            done = 0;
-        }
     }
 }
 
@@ -659,7 +631,6 @@ __device__ __forceinline__ void init_ring(const PairBars& br, int warps, int dep
             mbar_init(&br.full[d], 1);
             mbar_init(&br.empty[d], warps);
         }
-        br.ps->next[0] = br.ps->next[1] = kNoTarget;
         mbar_init_fence();
     }
     __syncthreads();
@@ -683,7 +654,7 @@ __global__ void __launch_bounds__(THREADS, blocks_per_sm(THREADS))
     __shared__ PlaneShared plane;
     const PairBars br{full_bar, empty_bar, hdr, &plane};
     init_ring(br, WARPS, kDepth);
-    RingState rs{0, 0, 0, false};
+    RingState rs{0, 0, false};
     auto& sm = *reinterpret_cast<PairSmem<WARPS, PSI>*>(smem_raw);
     if (PSI && threadIdx.x < 32) sm.lg[threadIdx.x] = log2(1.0 + threadIdx.x / 32.0);  // read after run_item's barriers
     const WorkItem it = items[blockIdx.x];

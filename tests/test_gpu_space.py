@@ -82,3 +82,26 @@ def test_a_few_off_the_sphere(fss, method, levels):
     s, a = points(900, 7)
     s[[3, 120, 121, 500, 899], :3] *= np.array([0.9, 1.1, 1 + 1e-12, 1.3, 1 - 1e-5])[:, None]
     check(fss, s, a, method, levels)
+
+
+def pair_time(ctx, s, a):
+    """Least device time of the pair sums of one right-hand side, of 8."""
+    times = []
+    for _ in range(8):
+        ctx.profile(True)
+        ctx.rhs(s, a)
+        times.append(ctx.profile_read()["pairs_fp64"][0])
+    return min(times)
+
+
+def test_a_tree_at_other_positions_takes_one_pass(fss):
+    """Leaves whose particles lie all over the sphere cost what a sum in space
+    costs (14 operations a pair for 10), not a pass over the sources for each
+    group of them, which takes three times a tree's own positions and more.
+    Twice is between the two."""
+    s, a = points(40962, 11)
+    t = s.copy()
+    t[:, :3] = s[np.random.default_rng(1).permutation(len(s)), :3]
+    with fss.Context(precision=fss.PREC_FP64) as c:
+        c.set_particles(s, a)
+        assert pair_time(c, t, a) < 2 * pair_time(c, s, a)
