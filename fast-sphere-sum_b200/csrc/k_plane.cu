@@ -1,5 +1,5 @@
 // k_plane.cu -- the FP64 pair engine: direct sum, near field and far field,
-// summed in the plane.
+// summed in the plane, what is near in space.
 //
 // A block works on one work item: the targets of one leaf (taken in chunks,
 // chunk_targets; the leaf's current particle range is read from leaf_start on
@@ -28,21 +28,25 @@
 // so that a pair costs 10 FP64 operations (2 differences, 2 for r^2, 4 for
 // w / r^2, 2 accumulations) where differences in space cost 14; everything
 // else is done once per source and chunk (about 40 operations) or once per
-// target.  The map keeps the relative precision of x - c near the targets, so
-// neighbours' differences carry the rounding of the positions and no more.
+// target.
 //
-// The map holds on the unit sphere alone and serves targets on c's side of it
+// A difference in the plane carries the map's rounding, a few u |xi| (u =
+// 2^-53), where one in space is exact for neighbours: relative to a pair h
+// apart, a few u |xi| / h.  So the plane takes only sources beyond kNear times
+// the targets' largest |xi|, each target at least a fifth of |xi_j| away.  And
+// the map holds on the unit sphere alone and serves targets on c's side of it
 // (kMinCos).  What it does not serve is summed in space, at 14 operations a
-// pair: a warp's share of a tile with a source off the sphere (kOnSphere), and
-// every share for a chunk with a target off it or with targets all over it
-// (a tree evaluated at other positions than its own: 163,842 particles 1.40 ms,
+// pair: sources near the targets or off the sphere (kOnSphere), and every
+// source for a chunk with a target off the sphere or with targets all over it
+// (a tree evaluated at other positions than its own: 163,842 particles 1.33 ms,
 // where a pass over the sources around each group of targets took 4.31).
 //
-// Bound by the FP64 pipe, 80% busy (20 of the 27 cycles that a pair takes a
-// warp).  Per right-hand side, before and now: treecode of 163,842 particles
-// (n = 8, theta = 0.7; 1.29e9 lane pairs) 1.347 and 0.918 ms; direct sum of
-// 20,011 particles 0.403 and 0.33 ms; 40,962 particles with the stream
-// function 1.18 and 0.48 ms.
+// Bound by the FP64 pipe.  Pair sums of one right-hand side, all in space by
+// one target a lane and here: treecode of 163,842 particles (n = 8, theta =
+// 0.7) 1.320 and 0.979 ms (0.929 with all sources but the targets in the
+// plane), with target clusters (n = 10) 0.760 and 0.594; direct sum of 20,011
+// particles 0.402 and 0.323; 40,962 particles with the stream function 1.156
+// and 0.492.
 // The FP32 engine (k_pairs.cu) sums in space.
 #include <algorithm>
 
@@ -56,7 +60,14 @@ constexpr int kTile = tile_capacity(true);
 constexpr double kMinCos = 0.2;  // the plane serves targets with x.c above this
 constexpr int kSlots = 32 * (kMaxFull + 1);  // accumulator slots of a warp
 
-// What the guarded pair loop adds to r^2, so that a source at the target's
+// Sources with |xi| up to this times the targets' largest (and to the distance
+// below which a position's rounding across the sphere would show) are near.
+// Direct sums of 2,001 to 163,842 random particles, plainly summed, come out to
+// 2.2e-16 to 5.2e-16 of the result with it as with 1.5, 2 and 3 (in space 8e-16
+// to 1.4e-14, in longer sums); the level-7 treecode above 0.979, at 1.5 0.996 ms.
+constexpr double kNear = 1.25;
+constexpr double kNearest = 1e-6;
+// What the pair loop in space adds to r^2, so that a source at the target's
 // position (r^2 = 0) has a finite reciprocal that multiplies a zero
 // difference; far below any other r^2.
 constexpr double kSelfR2 = 1e-200;
@@ -77,7 +88,8 @@ __device__ __forceinline__ bool on_sphere(double x, double y, double z) {
 // The plane of a chunk of targets, in shared memory.
 struct PlaneShared {
     double c[3], e1[3], e2[3];
-    int flat;  // it serves them
+    int flat;   // it serves them
+    int reach;  // the largest |xi|^2 of them (a float rounded up, its bits)
 };
 struct Plane {
     double c[3], a[3], b[3];
@@ -94,21 +106,15 @@ struct Plane {
     }
 };
 
-// Stereographic coordinates of a point near the unit sphere, put on it first
-// (two Newton steps for 1 / |x|: a position rounded to few digits must not be
-// moved along the sphere by its distance from it).  With t = x - c on c's
-// side, 1 + x.c = (4 - |t|^2) / 2; with t = x + c on the other, |t|^2 / 2 (and
-// x.e = t.e either way); close to the antipode -c, where t's radial part is
-// rounding, |t|^2 = 2 (1 - sqrt(1 - q)) with q = (t.e1)^2 + (t.e2)^2.
-// Explicitly rounded operations: a target and the same point as a source must
-// map to the same bits.
+// Stereographic coordinates of x / |x|, x on the sphere but for rounding: xi =
+// (x.e1, x.e2) / (|x| + x.c).  With t = x - c on c's side, |x| + x.c =
+// ((1 + |x|)^2 - |t|^2) / 2, and (1 + |x|)^2 = 2 + 2 |x|^2; with t = x + c on
+// the other, |t|^2 / 2 (and x.e = t.e either way); close to the antipode -c,
+// where t's radial part is rounding, |t|^2 = 2 (1 - sqrt(1 - q)) with q =
+// (t.e1)^2 + (t.e2)^2.  Explicitly rounded operations: a target and the same
+// point as a source map to the same bits, so that it is among the near.
 __device__ __forceinline__ void plane_map(const Plane& p, double x, double y, double z, double& u, double& v) {
     const double nn = norm2(x, y, z);
-    double n = __fma_rn(-0.5, nn, 1.5);
-    n = __dmul_rn(n, __fma_rn(__dmul_rn(-0.5, nn), __dmul_rn(n, n), 1.5));
-    x = __dmul_rn(x, n);
-    y = __dmul_rn(y, n);
-    z = __dmul_rn(z, n);
     const double dc = __fma_rn(z, p.c[2], __fma_rn(y, p.c[1], __dmul_rn(x, p.c[0])));
     const double s = -copysign(1.0, dc);
     const double tx = __fma_rn(s, p.c[0], x), ty = __fma_rn(s, p.c[1], y), tz = __fma_rn(s, p.c[2], z);
@@ -124,10 +130,11 @@ __device__ __forceinline__ void plane_map(const Plane& p, double x, double y, do
         v = away ? b * k : 0.0;
         return;
     }
-    const double k = rcp_fast(__dmul_rn(0.5, far ? tt : __dsub_rn(4.0, tt)));
+    const double k = rcp_fast(far ? __dmul_rn(0.5, tt) : __fma_rn(-0.5, tt, __dadd_rn(1.0, nn)));
     u = __dmul_rn(a, k);
     v = __dmul_rn(b, k);
 }
+__device__ __forceinline__ double rho_of(double u, double v) { return __fma_rn(v, v, __dmul_rn(u, u)); }
 
 // The plane around (x, y, z): c its direction, e1 and e2 by the branchless
 // construction of Duff et al., "Building an orthonormal basis, revisited"
@@ -168,8 +175,8 @@ struct Acc3 {
 // (P. T. P. Tang's table-driven logarithm, ACM TOMS 16, 1990, with a
 // reciprocal in place of a division as in W. F. Wong and E. Goto, IEEE Trans.
 // Computers 43, 1994).  About 12 FP64 operations where log2() took 75: the
-// sums with the stream function of 40,962 particles 1.18 ms with
-// log2(), 0.48 ms with this.
+// sums with the stream function of 40,962 particles 1.16 ms with
+// log2(), 0.49 ms with this.
 __device__ __forceinline__ double log2_beside(double r2, double y, const double* __restrict__ lg) {
     const int t = (__double2hiint(y) + 0x4000) & ~0x7fff;
     const double r = fma(r2, __hiloint2double(t, 0), -1.0);
@@ -186,22 +193,17 @@ __device__ __forceinline__ double log2_beside(double r2, double y, const double*
 
 // Pairs of NT targets of a lane with units (two sources, one 128-bit load per
 // component) q0, q0 + step, ... < q1 of mapped sources (arrays u, v, w of
-// SHARE entries, padded to whole units with w = 0).  A source at a target's
-// position must add nothing, also not to W.  GUARD (the tiles known to hold
-// the targets themselves): a bias on r^2 keeps its reciprocal finite, and its
-// w is summed into wz as (w / r^2) times the bias -- exact for it, nothing for
-// any other source.  Without GUARD its reciprocal is infinite and the sums
-// come out NaN, for which the caller takes the sources again, guarded.
+// SHARE entries, padded to whole units with w = 0), none of them near.
 //
 // The reciprocal is the hardware approximation y of 1 / r^2 (relative error
 // e < 2^-18) refined by y (1 + e + e^2), error e^3 < 2^-54, folded into the
 // product with w.
-template <bool PSI, bool GUARD, int SHARE, int NT>
+template <bool PSI, int SHARE, int NT>
 __device__ __forceinline__ void plane_pairs(const double* __restrict__ s, int q0, int q1, int step,
                                             const double2 (&t)[NT], double (&bu)[NT], double (&bv)[NT],
-                                            double (&wz)[NT], double (&ap)[NT], const double* __restrict__ lg) {
+                                            double (&ap)[NT], const double* __restrict__ lg) {
 #pragma unroll
-    for (int k = 0; k < NT; k++) bu[k] = bv[k] = wz[k] = ap[k] = 0.0;
+    for (int k = 0; k < NT; k++) bu[k] = bv[k] = ap[k] = 0.0;
 #pragma unroll(PSI ? 1 : (NT == 1 ? 4 : kUnroll))
     for (int q = q0; q < q1; q += step) {
         const double2 U = reinterpret_cast<const double2*>(s)[q];
@@ -213,19 +215,14 @@ __device__ __forceinline__ void plane_pairs(const double* __restrict__ s, int q0
 #pragma unroll
             for (int k = 0; k < NT; k++) {
                 const double du = qu[h] - t[k].x, dv = qv[h] - t[k].y;
-                const double r2 = fma(dv, dv, GUARD ? fma(du, du, kSelfR2) : du * du);
+                const double r2 = fma(dv, dv, du * du);
                 const double y = rcp_seed(r2);
                 const double e = fma(-r2, y, 1.0);
                 const double wy = qw[h] * y;
                 const double sc = fma(wy, fma(e, e, e), wy);
                 bu[k] = fma(sc, du, bu[k]);
                 bv[k] = fma(sc, dv, bv[k]);
-                if (GUARD) wz[k] = fma(sc, kSelfR2, wz[k]);
-                if (PSI) {
-                    double l = log2_beside(r2, y, lg);
-                    if (GUARD) l = (r2 > kSelfR2) ? l : 0.0;
-                    ap[k] = fma(qw[h], l, ap[k]);
-                }
+                if (PSI) ap[k] = fma(qw[h], log2_beside(r2, y, lg), ap[k]);
             }
     }
 }
@@ -233,29 +230,20 @@ __device__ __forceinline__ void plane_pairs(const double* __restrict__ s, int q0
 // A warp's share of a tile for its lanes' NT targets (positions tpos[32 k]),
 // added to the lane's accumulators.
 template <bool PSI, int SHARE, int NT>
-__device__ __forceinline__ void plane_fold(const double* __restrict__ share, int q0, int q1, int step, bool guard,
-                                           const double2* tpos, Acc* acc, double* accp, double* wz,
-                                           const double* lg) {
+__device__ __forceinline__ void plane_fold(const double* __restrict__ share, int q0, int q1, int step,
+                                           const double2* tpos, Acc* acc, double* accp, const double* lg) {
     const int lane = threadIdx.x & 31;
     double2 t[NT];
-    double bu[NT], bv[NT], bz[NT], bp[NT];
+    double bu[NT], bv[NT], bp[NT];
 #pragma unroll
     for (int k = 0; k < NT; k++) t[k] = tpos[32 * k];
-    if (!guard) {
-        plane_pairs<PSI, false, SHARE, NT>(share, q0, q1, step, t, bu, bv, bz, bp, lg);
-        bool bad = false;
-#pragma unroll
-        for (int k = 0; k < NT; k++) bad |= !(bu[k] - bu[k] == 0.0) || !(bv[k] - bv[k] == 0.0);
-        guard = __any_sync(0xffffffffu, bad);  // a source at a target's position (or a non-finite one)
-    }
-    if (guard) plane_pairs<PSI, true, SHARE, NT>(share, q0, q1, step, t, bu, bv, bz, bp, lg);
+    plane_pairs<PSI, SHARE, NT>(share, q0, q1, step, t, bu, bv, bp, lg);
 #pragma unroll
     for (int k = 0; k < NT; k++) {
         Acc& a = acc[32 * k + lane];
         a.u += bu[k];
         a.v += bv[k];
         if (PSI) accp[32 * k + lane] += bp[k];
-        if (guard) wz[32 * k + lane] += bz[k];
     }
 }
 
@@ -272,7 +260,7 @@ __device__ __forceinline__ void space_pairs(const double4* __restrict__ s, int j
         a[k] = Acc3{};
         ap[k] = 0.0;
     }
-#pragma unroll(PSI ? 1 : 2)
+#pragma unroll(PSI ? 2 : 4)
     for (int j = j0; j < n; j += step) {
         const double4 q = s[j];
 #pragma unroll
@@ -291,7 +279,7 @@ __device__ __forceinline__ void space_pairs(const double4* __restrict__ s, int j
     }
 }
 
-// A warp's share of a tile for its lanes' NT targets (tgt[32 k]) in space,
+// Such sources of a warp's share of a tile for its lanes' NT targets (tgt[32 k]),
 // added to the lane's accumulators.
 template <bool PSI, int NT>
 __device__ __forceinline__ void space_fold(const double4* __restrict__ share, int j0, int n, int step,
@@ -314,44 +302,58 @@ __device__ __forceinline__ void space_fold(const double4* __restrict__ share, in
     }
 }
 
-// A warp's share of a landed tile -- n sources from `in` -- mapped to the
-// plane (lane L takes sources L, L + 32, ...: conflict-free) into the warp's
-// own arrays u, v, w of SHARE entries, padded to whole units with w = 0; the
-// lane's sums of w and w log2(1 + rho) added to wsum and lsum.  False when a
-// source is not on the sphere: the share is to be summed in space (and
-// nothing is added).
+// A warp's share of a landed tile -- n sources, `in` -- parted: those that the
+// plane serves are mapped to it, into the warp's own arrays u, v, w of SHARE
+// entries, padded to whole units with w = 0 (nf of them, their sums of w and w
+// log2(1 + rho) added to wsum and lsum); those off the sphere or near the
+// targets (|xi|^2 <= near2) move to the front of `in` (nn of them).
 template <bool PSI, int SHARE>
-__device__ __forceinline__ bool map_share(const double4* __restrict__ in, double* __restrict__ out, int n,
-                                          const Plane& p, double& wsum, double& lsum) {
+__device__ __forceinline__ void part_share(double4* __restrict__ in, double* __restrict__ out, int n, const Plane& p,
+                                           double near2, int& nf, int& nn, double& wsum, double& lsum) {
+    constexpr int ROUNDS = (SHARE + 31) / 32;
     const int lane = threadIdx.x & 31;
-    const int padded = (n + 1) & ~1;
-    double ws = 0, ls = 0;
-    bool flat = true;
-#pragma unroll 2
-    for (int j = lane; j < padded; j += 32) {
-        double u = kFarAway, v = 0, w = 0;
-        if (j < n) {
-            const double4 q = in[j];
-            flat = flat && on_sphere(q.x, q.y, q.z);
-            plane_map(p, q.x, q.y, q.z, u, v);
-            w = q.w;
+    const unsigned below = (1u << lane) - 1;
+    double4 q[ROUNDS];
+#pragma unroll
+    for (int i = 0; i < ROUNDS; i++)
+        if (32 * i + lane < n) q[i] = in[32 * i + lane];
+    __syncwarp();  // all read before any is overwritten
+    nf = nn = 0;
+#pragma unroll
+    for (int i = 0; i < ROUNDS; i++) {
+        const bool any = 32 * i + lane < n;
+        double u = 0, v = 0;
+        bool far = false;
+        if (any) {
+            plane_map(p, q[i].x, q[i].y, q[i].z, u, v);
+            far = on_sphere(q[i].x, q[i].y, q[i].z) && rho_of(u, v) > near2;
         }
-        out[j] = u;
-        out[SHARE + j] = v;
-        out[2 * SHARE + j] = w;
-        ws += w;
-        if (PSI) ls += w * lg2_fast(fma(v, v, fma(u, u, 1.0)));
+        const unsigned fars = __ballot_sync(0xffffffffu, far), nears = __ballot_sync(0xffffffffu, any && !far);
+        if (far) {
+            const int k = nf + __popc(fars & below);
+            out[k] = u;
+            out[SHARE + k] = v;
+            out[2 * SHARE + k] = q[i].w;
+            wsum += q[i].w;
+            if (PSI) lsum += q[i].w * lg2_fast(fma(v, v, fma(u, u, 1.0)));
+        } else if (any) {
+            in[nn + __popc(nears & below)] = q[i];
+        }
+        nf += __popc(fars);
+        nn += __popc(nears);
     }
-    if (!__all_sync(0xffffffffu, flat)) return false;
-    wsum += ws;
-    if (PSI) lsum += ls;
-    return true;
+    if (lane == 0 && (nf & 1)) {
+        out[nf] = kFarAway;
+        out[SHARE + nf] = 0.0;
+        out[2 * SHARE + nf] = 0.0;
+    }
+    if (nn > 0) fence_proxy_async_smem();  // before the slot's next copy lands over them
 }
 
-// Tile header written by warp 0 before the slot's arrive (every warp reads it
-// after the slot's phase completes).
+// Tile header (sources) written by warp 0 before the slot's arrive (every warp
+// reads it after the slot's phase completes).
 struct SlotHdr {
-    int count, guard;
+    int count;
 };
 
 struct RingState {
@@ -362,9 +364,9 @@ struct RingState {
 // A target's A (and its log2 sum) from the sums in the plane.
 template <bool PSI>
 __device__ __forceinline__ double4 target_sum(const PlaneShared& ps, double wtot, double ltot, double x, double y, double z, double tu, double tv,
-                                              double bu, double bv, double bp, double wz) {
+                                              double bu, double bv, double bp) {
     const double u = tu, v = tv, rho = u * u + v * v;
-    const double W = wtot - wz, f = W / (1.0 + rho);
+    const double W = wtot, f = W / (1.0 + rho);
     const double p1 = bu + f * u, p2 = bv + f * v;
     const double g = 0.5 * (1.0 + rho), h = p1 * u + p2 * v;
     const double k1 = g * p1 - h * u, k2 = g * p2 - h * v, kx = 0.5 * W;
@@ -374,12 +376,12 @@ __device__ __forceinline__ double4 target_sum(const PlaneShared& ps, double wtot
     o.z = k1 * ps.e1[2] + k2 * ps.e2[2] - h * ps.c[2] - kx * z;
     o.w = 0.0;
     if (PSI)  // log2 |x_j - x_i|^2 = log2 |xi_j - xi_i|^2 + 2 - log2(1 + rho_i) - log2(1 + rho_j)
-        o.w = bp + W * (2.0 - log2(1.0 + rho)) - (ltot - wz * lg2_fast(fma(tv, tv, fma(tu, tu, 1.0))));
+        o.w = bp + W * (2.0 - log2(1.0 + rho)) - ltot;
     return o;
 }
 
 // Shared memory of a pair block: the landing ring (kDepth tiles as copied),
-// and each warp's mapped share of a tile, accumulators and sums over its
+// and each warp's parted share of a tile, accumulators and sums over its
 // sources; the targets' plane coordinates.
 template <int WARPS, bool PSI>
 struct PairSmem {
@@ -389,7 +391,6 @@ struct PairSmem {
     Acc acc[WARPS * kSlots];
     Acc3 acc3[WARPS * kSlots];
     double2 tpos[kSlots];
-    double wz[WARPS * kSlots];
     double accp[PSI ? WARPS * kSlots : 1];
     double wsum[WARPS], lsum[WARPS];
     double lg[PSI ? 32 : 1];  // log2(1 + i/32)
@@ -402,9 +403,9 @@ struct PairBars {
 
 // One work item: every chunk of targets against every tile of its segments.
 // Warp 0 packs and issues the tiles, one ahead of the one in use.  Every warp
-// maps its share of a landed tile to the plane, releases the slot through
-// empty (a share summed in space is read from the slot, which is released
-// after), and takes its share for all targets of the chunk: cn >> 5 targets a
+// parts its share of a landed tile, sums those in space from the slot, releases
+// it through empty, and sums those in the plane, each for all targets of the
+// chunk: cn >> 5 targets a
 // lane (a source loaded serves them all) and, for the r = cn & 31 left over,
 // L = 32 / r lanes a target, which split the share between them.  So the
 // warps' work is equal whatever the count of targets (one warp per 32 targets
@@ -449,12 +450,11 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                 // test hook: the first tile is neither copied nor signalled
                 if (lane == 0) br.hdr[slot].count = cnt;
             } else {
-                bool gd = false;
-                cnt = pack_tile<double4, kTile, true>(segs, leaf_start, it.g1, win, t0, t0 + nt, src, sm.ring + slot * kTile,
-                                          &br.full[slot], gd);
+                bool with_targets;  // (near shares need no telling)
+                cnt = pack_tile<double4, kTile, true>(segs, leaf_start, it.g1, win, t0, t0 + nt, src,
+                                                      sm.ring + slot * kTile, &br.full[slot], with_targets);
                 if (lane == 0) {
                     br.hdr[slot].count = cnt;
-                    br.hdr[slot].guard = gd ? 1 : 0;
                     mbar_arrive(&br.full[slot]);
                 }
             }
@@ -483,17 +483,16 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             if (lane == 0) {
                 plane_around(mx, my, mz, *ps);
                 ps->flat = 1;
+                ps->reach = 0;
             }
         }
         Acc* acc = sm.acc + warp * kSlots;
         Acc3* acc3 = sm.acc3 + warp * kSlots;
         double* accp = PSI ? sm.accp + warp * kSlots : sm.accp;
-        double* wz = sm.wz + warp * kSlots;
         double* mapped = sm.mapped + warp * 3 * SHARE;
         for (int k = lane; k < 32 * (full + 1); k += 32) {
             acc[k] = Acc{};
             acc3[k] = Acc3{};
-            wz[k] = 0;
             if (PSI) accp[k] = 0.0;
         }
         __syncthreads();
@@ -505,11 +504,15 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                 double2 p;
                 plane_map(plane, v.x, v.y, v.z, p.x, p.y);
                 sm.tpos[i] = p;
-                if (!on_sphere(v.x, v.y, v.z) || !plane.serves(v.x, v.y, v.z)) ps->flat = 0;
+                if (on_sphere(v.x, v.y, v.z) && plane.serves(v.x, v.y, v.z))
+                    atomicMax(&ps->reach, __float_as_int(__double2float_ru(rho_of(p.x, p.y))));
+                else
+                    ps->flat = 0;
             }
         }
         __syncthreads();
         const bool flat = ps->flat != 0;
+        const double near2 = fmax(kNear * kNear * double(__int_as_float(ps->reach)), kNearest * kNearest);
         double wsum = 0, lsum = 0;
         while (!rs.failed) {
             if (warp == 0 && !packed) {
@@ -525,46 +528,48 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             const SlotHdr h = br.hdr[slot];
             const int nu = (h.count + UNIT - 1) / UNIT;
             const int q0 = nu * warp / WARPS, q1 = nu * (warp + 1) / WARPS, nq = q1 - q0;
-            const double4* share = sm.ring + slot * kTile + q0 * UNIT;
+            double4* share = sm.ring + slot * kTile + q0 * UNIT;
             const int ns = min(h.count, q1 * UNIT) - q0 * UNIT;
-            bool space = nq > 0 && !flat;
-            if (nq > 0 && flat) {
+            int nf = 0, nn = 0;
+            if (flat) {
                 Plane plane;
                 plane.load(*ps);
-                space = !map_share<PSI, SHARE>(share, mapped, ns, plane, wsum, lsum);
+                part_share<PSI, SHARE>(share, mapped, ns, plane, near2, nf, nn, wsum, lsum);
+            } else if (nq > 0) {
+                nn = ns;
             }
-            if (space) {
+            __syncwarp();
+            if (nn > 0) {
                 const double4* tgt = src + t0 + c0;
                 int g = 0;
                 for (; g + 2 <= full; g += 2)
-                    space_fold<PSI, 2>(share, 0, ns, 1, tgt + 32 * g + lane, acc3 + 32 * g,
+                    space_fold<PSI, 2>(share, 0, nn, 1, tgt + 32 * g + lane, acc3 + 32 * g,
                                        PSI ? accp + 32 * g : accp, sm.lg);
                 if (g < full)
-                    space_fold<PSI, 1>(share, 0, ns, 1, tgt + 32 * g + lane, acc3 + 32 * g,
+                    space_fold<PSI, 1>(share, 0, nn, 1, tgt + 32 * g + lane, acc3 + 32 * g,
                                        PSI ? accp + 32 * g : accp, sm.lg);
                 if (r > 0)
-                    space_fold<PSI, 1>(share, lane % L, ns, L, tgt + 32 * full + min(lane / L, r - 1),
+                    space_fold<PSI, 1>(share, lane % L, nn, L, tgt + 32 * full + min(lane / L, r - 1),
                                        acc3 + 32 * full, PSI ? accp + 32 * full : accp, sm.lg);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&br.empty[slot]);
             rs.taken++;
             if (h.count == 0) break;
-            if (nq > 0 && !space) {
-                const bool gd = h.guard != 0;
+            if (nf > 0) {
+                const int nu = (nf + UNIT - 1) / UNIT;
                 const auto* tp = sm.tpos + lane;
                 switch (full) {
-                    case 1: plane_fold<PSI, SHARE, 1>(mapped, 0, nq, 1, gd, tp, acc, accp, wz, sm.lg); break;
-                    case 2: plane_fold<PSI, SHARE, 2>(mapped, 0, nq, 1, gd, tp, acc, accp, wz, sm.lg); break;
-                    case 3: plane_fold<PSI, SHARE, 3>(mapped, 0, nq, 1, gd, tp, acc, accp, wz, sm.lg); break;
-                    case 4: plane_fold<PSI, SHARE, 4>(mapped, 0, nq, 1, gd, tp, acc, accp, wz, sm.lg); break;
+                    case 1: plane_fold<PSI, SHARE, 1>(mapped, 0, nu, 1, tp, acc, accp, sm.lg); break;
+                    case 2: plane_fold<PSI, SHARE, 2>(mapped, 0, nu, 1, tp, acc, accp, sm.lg); break;
+                    case 3: plane_fold<PSI, SHARE, 3>(mapped, 0, nu, 1, tp, acc, accp, sm.lg); break;
+                    case 4: plane_fold<PSI, SHARE, 4>(mapped, 0, nu, 1, tp, acc, accp, sm.lg); break;
                 }
                 if (r > 0)
-                    plane_fold<PSI, SHARE, 1>(mapped, lane % L, nq, L, gd, sm.tpos + 32 * full + min(lane / L, r - 1),
-                                                acc + 32 * full, PSI ? accp + 32 * full : accp, wz + 32 * full,
-                                             sm.lg);
-                __syncwarp();  // the share is used up before the next one is mapped over it
+                    plane_fold<PSI, SHARE, 1>(mapped, lane % L, nu, L, sm.tpos + 32 * full + min(lane / L, r - 1),
+                                              acc + 32 * full, PSI ? accp + 32 * full : accp, sm.lg);
             }
+            __syncwarp();  // the share is used up before the next one takes its place
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -594,7 +599,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             const double x = v.x, y = v.y, z = v.z;
             const bool rest = tgt >= 32 * full;
             const int s0 = rest ? 32 * full + L * (tgt - 32 * full) : tgt, ns = rest ? L : 1;
-            double bu = 0, bv = 0, bp = 0, bz = 0, wtot = 0, ltot = 0;
+            double bu = 0, bv = 0, bp = 0, wtot = 0, ltot = 0;
             Acc3 in_space{};
             for (int w = 0; w < WARPS; w++) {
                 wtot += sm.wsum[w];
@@ -607,14 +612,13 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                     in_space.x += a3.x;
                     in_space.y += a3.y;
                     in_space.z += a3.z;
-                    bz += sm.wz[w * kSlots + k];
                     if (PSI) bp += sm.accp[w * kSlots + k];
                 }
             }
             double4 o = make_double4(0.0, 0.0, 0.0, bp);
             if (flat) {
                 const double2 p = sm.tpos[tgt];
-                o = target_sum<PSI>(*ps, wtot, ltot, x, y, z, p.x, p.y, bu, bv, bp, bz);
+                o = target_sum<PSI>(*ps, wtot, ltot, x, y, z, p.x, p.y, bu, bv, bp);
             }
             o.x += in_space.x;
             o.y += in_space.y;
@@ -637,8 +641,7 @@ __device__ __forceinline__ void init_ring(const PairBars& br, int warps, int dep
 }
 
 // Blocks per SM that the registers must allow: 128 a thread, four blocks of
-// four warps (at 96 and five blocks the level-7 treecode took 0.958 ms per
-// right-hand side instead of 0.939).
+// four warps, as many as the shared memory holds.
 constexpr int blocks_per_sm(int threads) { return 65536 / 128 / threads; }
 
 // One block per work item; a ring of kDepth tile slots.

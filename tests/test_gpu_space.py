@@ -84,6 +84,28 @@ def test_a_few_off_the_sphere(fss, method, levels):
     check(fss, s, a, method, levels)
 
 
+@pytest.mark.parametrize("method,levels", ALL_PAIRS + [(1, 3)])
+@pytest.mark.parametrize("h", [1e-2, 1e-3, 1e-4, 1e-6, 1e-8])
+def test_close_pairs(fss, h, method, levels):
+    """Pairs h apart, of opposite weights, wherever in their leaf they lie."""
+    s, a = points(1200, 9)
+    near = s[:600, :3] + h * np.random.default_rng(2).standard_normal((600, 3))
+    s[600:, :3] = near / np.linalg.norm(near, axis=1, keepdims=True)
+    s[600:, 3] = -s[:600, 3]
+    check(fss, s, a, method, levels)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 33, 64, 127, 129, 160, 161, 300])
+def test_one_region(fss, n):
+    """Particles of a region that one plane serves, among others far away: every
+    count of near and far sources in a warp's share."""
+    s, a = points(n + 500, n)
+    s[:n, :3] = np.array([1.0, 0.5, 0.2]) + 0.1 * s[:n, :3]
+    s[:n, :3] /= np.linalg.norm(s[:n, :3], axis=1, keepdims=True)
+    check(fss, s, a, 0, 0)
+    check(fss, s, a, 1, 2)
+
+
 def pair_time(ctx, s, a):
     """Least device time of the pair sums of one right-hand side, of 8."""
     times = []
