@@ -228,7 +228,7 @@ int build_direct_lists(fss_ctx* c) {
         nt = std::min<int64_t>(c->fp64 ? TB : direct_group(t_end - t_first, t0 - t_first, P), t_end - t0);
         for (int p = 0; p < P; p++) {
             L.items.push_back(WorkItem{int32_t(t0), int32_t(nt), p, p + 1, p, -1,
-                                       pair_split(double(L.segs[p].b - L.segs[p].a), int(nt), 4), 0});
+                                       pair_split(double(L.segs[p].b - L.segs[p].a), int(nt), c->shape.warps()), 0});
             L.n_tiles += (L.segs[p].b - L.segs[p].a + c->shape.tile - 1) / c->shape.tile;
         }
     }
@@ -606,6 +606,7 @@ int materialize(fss_ctx* c, PairShape shape) {
     in.parts = P;
     if (!c->fp64 && !c->member) leaf_group(c, P, in);
     c->shape.max_targets = in.group > 0 ? std::min(maxleaf, in.group + in.group / 2) : maxleaf;
+    in.leaf_warps = c->shape.warps();
     in.cluster_warps = cluster_shape(c->fp64, int64_t(c->tlists.size()) * P).warps();
     in.all_leaves = c->resort;
     c->parts = P;
@@ -871,9 +872,10 @@ int tune_rhs(fss_ctx* c) {
 // (leaf size), when the configuration leaves it automatic -- the automatic
 // depth and one level either side, each built and timed on a whole
 // right-hand side (the fastest is kept for this particle count); and the
-// source split (src_parts 1, 2, 4), when automatic, timed on a whole
-// right-hand side (more parts balance the pair launches but add partial
-// slots for the epilogue to sum).
+// source split (src_parts 1, 2, 4 and, in FP64, whose automatic split goes
+// further, that one and its neighbours), when automatic, timed on a whole
+// right-hand side (more parts balance the pair launches but add partial slots
+// for the epilogue to sum).
 // depth = false (lists rebuilt for per-leaf parameters, which belong to the
 // current leaves) keeps the tree.
 int autotune(fss_ctx* c, bool depth) {
@@ -928,7 +930,11 @@ int autotune(fss_ctx* c, bool depth) {
         c->tuned_parts.clear();
         int best_p = 1;
         double best_p_ms = 1e30;
-        for (int p : {1, 2, 4}) {
+        std::vector<int> splits = {1, 2, 4};
+        if (c->fp64)
+            for (int p = c->parts - 1; p <= c->parts + 1; p++)  // around the automatic split, in use here
+                if (p >= 1 && std::find(splits.begin(), splits.end(), p) == splits.end()) splits.push_back(p);
+        for (int p : splits) {
             c->cfg.src_parts = p;
             TRY(materialize(c, best));
             TRY(refresh_stage(c));

@@ -323,7 +323,7 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
                 const bool last = s + 1 == subs;
                 const int32_t first = s * grp, nt = last ? nt_est - first : grp;
                 items.push_back({w * nt, WorkItem{t0 + first, last ? nt_item : grp, base, g1, p, leaf,
-                                                  pair_split(w, nt, leaf >= 0 ? 4 : in.cluster_warps), 0}});
+                                                  pair_split(w, nt, leaf >= 0 ? in.leaf_warps : in.cluster_warps), 0}});
             }
         }
     };

@@ -109,7 +109,9 @@ typedef struct fss_config {
                               automatic depth and one level either side, each
                               timed on a whole right-hand side, the fastest kept
                               for this particle count) and, when src_parts is
-                              0, the source split (1, 2, 4: the fastest kept) */
+                              0, the source split (1, 2, 4 and, in FP64, the
+                              automatic split and the two next to it: the
+                              fastest kept) */
     int32_t rebuild;       /* fss_rebuild_policy */
     int32_t cluster_targets; /* 1 = the reference's cp/cc interaction types
                               (fast_rhs.h cp, cc): a well-separated target face

@@ -116,3 +116,28 @@ def test_autotune_depth_and_split(fss, oracle):
     assert info["src_parts"] in (1, 2, 4)
     assert again["tree_levels"] == info["tree_levels"]
     assert rel_l2(out[rows, :3], ref) < 1e-6
+
+
+@pytest.mark.parametrize("n,levels", [(2562, 1), (10242, 2), (20011, 2)])
+def test_autotune_fp64_split_is_no_slower(fss, n, levels):
+    """autotune = 2 in FP64 tries the automatic split too, so that tuning costs
+    no speed: within 6% of the untuned right-hand side (the candidates' timings
+    differ by 2 to 3% from run to run), where trying 1, 2 and 4 parts alone lost
+    15% of it on 20 leaves of 128 and on 80 of 250."""
+    rng = np.random.default_rng(3)
+    s = np.zeros((n, 5))
+    s[:, :3] = rng.standard_normal((n, 3))
+    s[:, :3] /= np.linalg.norm(s[:, :3], axis=1, keepdims=True)
+    s[:, 3] = rng.standard_normal(n)
+    a = np.full(n, 4 * np.pi / n)
+    ms = []
+    for tune in (0, 2):
+        with fss.Context(precision=fss.PREC_FP64, tree_levels=levels, autotune=tune) as ctx:
+            ctx.set_particles(s, a)
+            runs = []
+            for _ in range(20):
+                ctx.profile(True)
+                ctx.rhs_current()
+                runs.append(sum(v[0] for v in ctx.profile_read().values()))
+            ms.append(min(runs))
+    assert ms[1] < 1.06 * ms[0]
