@@ -665,6 +665,22 @@ int materialize(fss_ctx* c, PairShape shape) {
         std::vector<int32_t> index;
         c->up_per_block = batch_tasks(int64_t(up.size()));
         make_task_blocks(up, c->up_per_block, blocks, index);
+        // The blocks with the most to do first: by degree, the largest matrices come
+        // last, and with them blocks of coarse faces, which have 64 rows a moment
+        // to sum where others have 1 or 4. Upward combine of 655,362 particles with
+        // target clusters, us per right-hand side in that order and in this: learned
+        // degrees 56.7 39.4, of 4 to 10 at random 70.0 51.5, one degree 25.1 25.1.
+        std::stable_sort(blocks.begin(), blocks.end(), [&](const TaskBlock& a, const TaskBlock& b) {
+            auto cost = [&](const TaskBlock& t) {
+                int64_t rows = 0;
+                for (int32_t k = t.first; k < t.first + t.count; k++) {
+                    const ProxyJob& j = L.jobs[size_t(index[size_t(k)])];
+                    rows += (j.leaf_hi - j.leaf_lo + 3) / 4;
+                }
+                return nproxy(t.deg) * (rows + nproxy(t.deg));
+            };
+            return cost(a) > cost(b);
+        });
         c->n_up_blocks = int(blocks.size());
         TRY(upload(c, c->up_tblocks, blocks));
         TRY(upload(c, c->up_tasks, index));

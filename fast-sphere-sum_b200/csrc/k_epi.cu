@@ -88,10 +88,10 @@ static_assert((batch_pad(kMaxK) / 2) * 4 <= kBatchThreads, "one tile per thread 
 // Vinv[m][k] M_m of every (face, degree) task, written with the proxy
 // positions at the face's slots of the unified source array (absolute
 // coordinates).  Shared memory: A[m][k] = Vinv[m][k] (K rows of Kp; one bulk
-// copy of the padded matrix `vpad`), then X[t][m] = the task's moments.  The
-// rows were summed by a launch of their own, 4 to 7 us of latency that only a
-// face of several degrees made up for: with learned parameters at 655,362
-// particles the two took 13 + 37 us and this takes 52.
+// copy of the padded matrix `vpad`), then X[t][m] = the task's moments.  A
+// launch of their own for the rows, once per face instead of once per degree of
+// it, is slower whatever the degrees: 51.2 us against 39.4 with learned ones at
+// 655,362 particles, 12.3 against 8.4 with one degree at 40,962.
 template <typename T, int TT>
 __global__ void __launch_bounds__(kBatchThreads) k_up_proxies(const TaskBlock* __restrict__ blocks,
                                                               const int32_t* __restrict__ tasks,
