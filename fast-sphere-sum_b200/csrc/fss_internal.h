@@ -40,7 +40,7 @@ struct WorkItem {
     int32_t part;
     int32_t leaf;
     int32_t split;  // FP32: subsets of the targets that different warps sum
-    int32_t pad;
+    int32_t space;  // FP64: the targets are not near one another (no plane serves them)
 };
 
 // Targets of a work item that one pass of a pair block serves: up to kMaxFull

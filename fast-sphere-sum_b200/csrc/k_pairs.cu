@@ -142,17 +142,6 @@ __device__ __forceinline__ void kahan_add(float& sum, float& comp, float x) {
     sum = t;
 }
 
-// Sum over the L lanes of each group [L t, L t + L) of the warp (segmented
-// tree of shuffles, L warp-uniform); the group's first lane (sub = 0) holds
-// the sum.
-__device__ __forceinline__ float group_sum(float x, int sub, int L) {
-    for (int off = 1; off < L; off <<= 1) {
-        const float y = __shfl_down_sync(0xffffffffu, x, off);
-        if (sub + off < L) x += y;
-    }
-    return x;
-}
-
 // Turns of the warps at the totals, in the order of the tiles.
 __device__ __forceinline__ int turn_load(const int* p) {
     int v;

@@ -37,7 +37,8 @@
 // the map holds on the unit sphere alone and serves targets on c's side of it
 // (kMinCos).  What it does not serve is summed in space, at 14 operations a
 // pair: sources near the targets or off the sphere (kOnSphere), and every
-// source for a chunk with a target off the sphere or with targets all over it
+// source for a chunk with a target off the sphere or with targets all over it,
+// or of a direct sum in the caller's order (WorkItem::space)
 // (a tree evaluated at other positions than its own: 163,842 particles 1.33 ms,
 // where a pass over the sources around each group of targets took 4.31).
 //
@@ -468,7 +469,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
         } else if (warp == 1) {
             // c: the direction of the chunk's targets' mean
             double mx = 0, my = 0, mz = 0;
-            for (int i = lane; i < cn; i += 32) {
+            for (int i = lane; i < cn && !it.space; i += 32) {
                 const double4 v = src[t0 + c0 + i];
                 mx += v.x;
                 my += v.y;
@@ -482,7 +483,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             }
             if (lane == 0) {
                 plane_around(mx, my, mz, *ps);
-                ps->flat = 1;
+                ps->flat = !it.space;
                 ps->reach = 0;
             }
         }
@@ -496,7 +497,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             if (PSI) accp[k] = 0.0;
         }
         __syncthreads();
-        {
+        if (!it.space) {
             Plane plane;
             plane.load(*ps);
             for (int i = tid; i < cn; i += 32 * WARPS) {
@@ -580,6 +581,17 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
             sm.wsum[warp] = wsum;
             sm.lsum[warp] = lsum;
         }
+        if (r > 0 && L > 1) {  // the lanes of a target left over: their sums to the first of them
+            Acc& a = acc[32 * full + lane];
+            Acc3& a3 = acc3[32 * full + lane];
+            const int sub = lane % L;
+            a.u = group_sum(a.u, sub, L);
+            a.v = group_sum(a.v, sub, L);
+            a3.x = group_sum(a3.x, sub, L);
+            a3.y = group_sum(a3.y, sub, L);
+            a3.z = group_sum(a3.z, sub, L);
+            if (PSI) accp[32 * full + lane] = group_sum(accp[32 * full + lane], sub, L);
+        }
         if (warp > 0) rs.issued = rs.taken;
         // every tile issued for this chunk has been taken, so the counters
         // agree in every warp unless a wait gave up
@@ -593,27 +605,24 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                     mbar_wait_bounded(&br.full[t % kDepth], uint32_t(t / kDepth) & 1, ctl.wait_ns);
             return;
         }
-        // the targets' sums over the warps (and lanes)
+        // the targets' sums over the warps
         for (int tgt = tid; tgt < cn; tgt += 32 * WARPS) {
             const double4 v = src[t0 + c0 + tgt];
             const double x = v.x, y = v.y, z = v.z;
-            const bool rest = tgt >= 32 * full;
-            const int s0 = rest ? 32 * full + L * (tgt - 32 * full) : tgt, ns = rest ? L : 1;
+            const int k = tgt >= 32 * full ? 32 * full + L * (tgt - 32 * full) : tgt;
             double bu = 0, bv = 0, bp = 0, wtot = 0, ltot = 0;
             Acc3 in_space{};
             for (int w = 0; w < WARPS; w++) {
                 wtot += sm.wsum[w];
                 ltot += sm.lsum[w];
-                for (int k = s0; k < s0 + ns; k++) {
-                    const Acc& a = sm.acc[w * kSlots + k];
-                    bu += a.u;
-                    bv += a.v;
-                    const Acc3& a3 = sm.acc3[w * kSlots + k];
-                    in_space.x += a3.x;
-                    in_space.y += a3.y;
-                    in_space.z += a3.z;
-                    if (PSI) bp += sm.accp[w * kSlots + k];
-                }
+                const Acc& a = sm.acc[w * kSlots + k];
+                bu += a.u;
+                bv += a.v;
+                const Acc3& a3 = sm.acc3[w * kSlots + k];
+                in_space.x += a3.x;
+                in_space.y += a3.y;
+                in_space.z += a3.z;
+                if (PSI) bp += sm.accp[w * kSlots + k];
             }
             double4 o = make_double4(0.0, 0.0, 0.0, bp);
             if (flat) {

@@ -274,22 +274,20 @@ __global__ void k_gather(int64_t n, const double* __restrict__ in5, const double
 
 // ---------------------------------------------------------------- FP64 direct sum's order
 
-// The FP64 direct sum keeps its state in the caller's order; its sources (and
-// with them the blocks of targets and their partial sums) are laid out in a
-// spatial order, since a block serves targets near one another in one pass.
-// The order is that of the cells of a cube around the sphere, Morton order
+// The FP64 direct sum of many particles keeps its state in the caller's order;
+// its sources (and with them the blocks of targets and their partial sums) are
+// laid out in a spatial order, since a plane serves targets near one another.
+// The order is that of 24,576 cells of a cube around the sphere, Morton order
 // within a face, caller's order within a cell: a function of the positions
-// alone.  kOrderFew particles or fewer take 96 cells and one block that does
-// it all (642 particles: five launches made the right-hand side 10 us longer
-// than this one does); more take 24,576 and two radix passes.
-constexpr int kOrderFew = 4096, kFewCells = 96;
+// alone.
+constexpr int kLogSide = 6;  // cells along a face's edge
 __device__ __forceinline__ uint32_t spread_bits(uint32_t v) {  // bit i to bit 2 i (6 bits)
     uint32_t r = 0;
 #pragma unroll
     for (int i = 0; i < 6; i++) r |= ((v >> i) & 1u) << (2 * i);
     return r;
 }
-__device__ __forceinline__ uint32_t order_cell(const double4& p, int log_side) {
+__device__ __forceinline__ uint32_t order_cell(const double4& p) {
     const double ax = fabs(p.x), ay = fabs(p.y), az = fabs(p.z);
     // faces in the order +x, +y, -x, -y around the equator, then +z, -z
     int face = p.x >= 0 ? 0 : 2;
@@ -304,20 +302,20 @@ __device__ __forceinline__ uint32_t order_cell(const double4& p, int log_side) {
         a = p.x;
         b = p.y;
     }
-    const int side = 1 << log_side;
+    constexpr int side = 1 << kLogSide;
     // (a non-finite position lands in some cell)
     const int ia = min(side - 1, max(0, int((a / m + 1.0) * (0.5 * side))));
     const int ib = min(side - 1, max(0, int((b / m + 1.0) * (0.5 * side))));
-    return (uint32_t(face) << (2 * log_side)) | spread_bits(uint32_t(ia)) | (spread_bits(uint32_t(ib)) << 1);
+    return (uint32_t(face) << (2 * kLogSide)) | spread_bits(uint32_t(ia)) | (spread_bits(uint32_t(ib)) << 1);
 }
 
 __device__ __forceinline__ double4 source_of(const double4& v, double area) {
     return make_double4(v.x, v.y, v.z, v.w * area);
 }
 
-__global__ void k_order_keys(int64_t n, const double4* __restrict__ xs, int log_side, uint32_t* __restrict__ key) {
+__global__ void k_order_keys(int64_t n, const double4* __restrict__ xs, uint32_t* __restrict__ key) {
     const int64_t s = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (s < n) key[s] = order_cell(xs[s], log_side);
+    if (s < n) key[s] = order_cell(xs[s]);
 }
 
 // Sources in the order from the stage state.
@@ -327,72 +325,6 @@ __global__ void k_order_src(int64_t n, const int32_t* __restrict__ order, const 
     if (s >= n) return;
     const int64_t k = order[s];
     src[s] = source_of(xs[k], area[k]);
-}
-
-// Order and sources of up to kOrderFew particles, one block: a counting sort
-// in which warp w ranks particles [w m, (w + 1) m), so that it is stable.
-__global__ void __launch_bounds__(1024) k_order_few(int n, const double4* __restrict__ xs,
-                                                    const double* __restrict__ area, int32_t* __restrict__ order,
-                                                    double4* __restrict__ src) {
-    constexpr int kRounds = kOrderFew / 1024;
-    __shared__ int count[32][kFewCells];  // per warp, then its first slot per cell
-    __shared__ int total[kFewCells];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int m = 32 * ((n + 1023) / 1024);
-    for (int c = lane; c < kFewCells; c += 32) count[w][c] = 0;
-    __syncwarp();
-    double4 v[kRounds];
-    int cell[kRounds], rank[kRounds];
-#pragma unroll
-    for (int r = 0; r < kRounds; r++) {
-        const int i = w * m + 32 * r + lane;
-        const bool mine = 32 * r < m && i < n;
-        cell[r] = -1;
-        rank[r] = 0;
-        if (mine) {
-            v[r] = xs[i];
-            cell[r] = int(order_cell(v[r], 2));
-        }
-        const unsigned peers = __match_any_sync(0xffffffffu, cell[r]);
-        if (mine) rank[r] = count[w][cell[r]] + __popc(peers & ((1u << lane) - 1));
-        __syncwarp();
-        if (mine && (peers & ((1u << lane) - 1)) == 0) count[w][cell[r]] += __popc(peers);
-        __syncwarp();
-    }
-    __syncthreads();
-    if (threadIdx.x < kFewCells) {
-        int sum = 0;
-        for (int k = 0; k < 32; k++) {
-            const int c = count[k][threadIdx.x];
-            count[k][threadIdx.x] = sum;
-            sum += c;
-        }
-        total[threadIdx.x] = sum;
-    }
-    __syncthreads();
-    if (w == 0) {  // first slots of the cells
-        int base = 0;
-        for (int c0 = 0; c0 < kFewCells; c0 += 32) {
-            const int c = total[c0 + lane];
-            int incl = c;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += y;
-            }
-            total[c0 + lane] = base + incl - c;
-            base += __shfl_sync(0xffffffffu, incl, 31);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < kRounds; r++) {
-        if (cell[r] < 0) continue;
-        const int i = w * m + 32 * r + lane;
-        const int s = total[cell[r]] + count[w][cell[r]] + rank[r];
-        order[s] = i;
-        src[s] = source_of(v[r], area[i]);
-    }
 }
 
 // ---------------------------------------------------------------- re-sort
@@ -812,17 +744,13 @@ void launch_sort(cudaStream_t st, int64_t n, int bits, uint32_t* keys, uint32_t*
     if (vi != vals) cudaMemcpyAsync(vals, vi, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, st);
 }
 
-int order_launch_count(int64_t n) { return n <= kOrderFew ? 1 : 2 + sort_launch_count(n, 15); }
+int order_launch_count(int64_t n) { return 2 + sort_launch_count(n, 15); }
 
 void launch_order(cudaStream_t st, int64_t n, const double4* xs, const double* area, uint32_t* key,
                   uint32_t* key_tmp, int32_t* order, int32_t* vals_tmp, uint32_t* hist, double4* src) {
     if (n == 0) return;
-    if (n <= kOrderFew) {
-        k_order_few<<<1, 1024, 0, st>>>(int(n), xs, area, order, src);
-        return;
-    }
     const unsigned g = unsigned((n + 255) / 256);
-    k_order_keys<<<g, 256, 0, st>>>(n, xs, 6, key);
+    k_order_keys<<<g, 256, 0, st>>>(n, xs, key);
     launch_sort(st, n, 15, key, key_tmp, order, vals_tmp, hist);
     k_order_src<<<g, 256, 0, st>>>(n, order, xs, area, src);
 }

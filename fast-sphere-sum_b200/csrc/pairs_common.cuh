@@ -85,6 +85,18 @@ __device__ __forceinline__ int pack_tile(const Segment* __restrict__ segs, const
     return count;
 }
 
+// Sum over the L lanes of each group [L t, L t + L) of the warp (segmented
+// tree of shuffles, L warp-uniform); the group's first lane (sub = 0) holds
+// the sum.
+template <typename T>
+__device__ __forceinline__ T group_sum(T x, int sub, int L) {
+    for (int off = 1; off < L; off <<= 1) {
+        const T y = __shfl_down_sync(0xffffffffu, x, off);
+        if (sub + off < L) x += y;
+    }
+    return x;
+}
+
 // Dynamic shared memory above the default limit has to be allowed, on every
 // device that launches the kernel.
 template <typename K>

@@ -127,3 +127,39 @@ def test_a_tree_at_other_positions_takes_one_pass(fss):
     with fss.Context(precision=fss.PREC_FP64) as c:
         c.set_particles(s, a)
         assert pair_time(c, t, a) < 2 * pair_time(c, s, a)
+
+
+@pytest.mark.parametrize("n", [15000, 15001])
+def test_direct_order_only_where_it_pays(fss, n):
+    """Up to 15,000 particles the direct sum keeps the caller's order (the
+    spatial one takes eight launches a step, which cost 6,000 particles a third
+    more); beyond, the sums come out the same from the spatial order."""
+    s, a = points(n, 13)
+    x, w = s[:, :3].astype(np.longdouble), (s[:, 3] * a).astype(np.longdouble)
+    with fss.Context(method=fss.METHOD_DIRECT, precision=fss.PREC_FP64) as c:
+        c.set_particles(s, a)
+        out = c.rhs(s, a)
+        c.profile(True)
+        c.rk4_step(0.01)
+        assert ("order" in c.profile_read()) == (n > 15000)
+    for i in (0, 1, n // 2, n - 2, n - 1):
+        d = x - x[i]
+        r2 = (d * d).sum(1)
+        r2[i] = 1
+        f = w / r2
+        u = -np.cross(x[i], f @ d) / (2 * np.pi)
+        assert np.linalg.norm(out[i, :3] - u) <= (n + 32) * 2.0 ** -53 * (np.abs(f) * np.sqrt(r2)).sum() / (2 * np.pi)
+
+
+def test_ordered_direct_steps_resume_bit_for_bit(fss):
+    s, a = points(15600, 17)
+    with fss.Context(method=fss.METHOD_DIRECT, precision=fss.PREC_FP64) as c:
+        c.set_particles(s, a)
+        c.rk4_step(0.01)
+        mid = c.get_state()
+        c.rk4_step(0.01)
+        end = c.get_state()
+    with fss.Context(method=fss.METHOD_DIRECT, precision=fss.PREC_FP64) as c:
+        c.set_particles(mid, a)
+        c.rk4_step(0.01)
+        assert np.array_equal(c.get_state(), end)
