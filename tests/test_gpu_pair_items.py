@@ -86,3 +86,23 @@ def test_direct_uneven_items(fss):
         out, p = c.rhs(s, a, psi=True)
     assert np.all(np.linalg.norm(out[rows, :3] - u, axis=1) <= 8e-6 * mu)
     assert np.all(np.abs(p[rows] - psi) <= 8e-6 * mp)
+
+
+def pair_ms(ctx, psi=False):
+    times = []
+    for _ in range(10):
+        ctx.profile(True)
+        ctx.rhs_current(psi=psi)
+        times.append(ctx.profile_read()["pairs_mixed"][0])
+    return min(times)
+
+
+@pytest.mark.parametrize("clusters", [0, 1])
+def test_stream_function_costs_its_logarithm(fss, clusters):
+    """A logarithm a pair makes the sums 1.3 times as long (two operations of the
+    pipe that the reciprocal needs instead of one); with its loop unrolled eight
+    times it was 1.6 to 1.7 times."""
+    s, a = spread(163842, 3)
+    with fss.Context(cluster_targets=clusters) as c:
+        c.set_particles(s, a)
+        assert pair_ms(c, True) < 1.47 * pair_ms(c)
