@@ -174,21 +174,22 @@ int plane_parts(double blocks, double sources, int most) {
 // target t0 of n.  An item's targets are summed on their own, so the choice
 // changes no result.  256 (a block's most) in whole rounds of the 740 blocks
 // that run at once, the rest in 128s and then 64s, so that the last round ends
-// evenly; fewer targets than a round in 128s, 64s or 32s.  Measured, us per
-// right-hand side: in 128s, 64s, 32s 700 particles 19.0 15.2 12.7; 2,001 19.5
-// 15.1 14.6; 5,000 24.2 22.4 27.7; with all in 256s, and the rest in 128s, in
-// 64s, in both: 10,001 60.0 54.2 53.5 54.1; 14,982 103.6 99.1 99.4
-// 99.5; 20,011 175.3 173.9 167.6 166.8; 32,000 409 405 397 395; 60,000 1396
-// 1368 1342 1338.
+// evenly; fewer targets than a round in the smallest of 32s, 64s and 128s that
+// stay within one, as long as 128s do not fill it by themselves.  Measured, us
+// per RK4 step: in 128s, 64s, 32s 700 particles 64.2 54.0 41.4; 2,001 70.4 52.7
+// 50.5; 3,500 78.7 65.1 68.2; 3,700 73.8 62.3 83.9; 5,000 93.0 84.7 112; 6,000 112
+// 107; 7,000 (715 items of 128) 125.6 135.8; 9,000 192 200; us per right-hand
+// side with all in 256s, and the rest in 128s, in 64s, in both: 10,001 60.0 54.2
+// 53.5 54.1; 14,982 103.6 99.1 99.4 99.5; 20,011 175.3 173.9 167.6 166.8; 32,000
+// 409 405 397 395; 60,000 1396 1368 1342 1338.
 int64_t direct_group(int64_t n, int64_t t0, int parts) {
     auto items = [&](int64_t g) { return (n + g - 1) / g * parts; };
     if (items(256) >= 740) {
         const int64_t whole = n / 256 * parts / 740 * 740 / parts * 256;
         return t0 < whole ? 256 : (t0 < (whole + n) / 2 ? 128 : 64);
     }
-    if (items(128) >= 740) return 128;
-    if (items(64) >= 500) return 64;
-    return 32;
+    if (items(128) >= 700) return 128;
+    return items(32) > 740 ? 64 : 32;
 }
 
 // The FP64 direct sum of more than kOrderFrom particles lays them out in a

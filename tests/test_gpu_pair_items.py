@@ -106,3 +106,18 @@ def test_stream_function_costs_its_logarithm(fss, clusters):
     with fss.Context(cluster_targets=clusters) as c:
         c.set_particles(s, a)
         assert pair_ms(c, True) < 1.47 * pair_ms(c)
+
+
+def test_direct_items_fit_one_round(fss):
+    """3,700 particles in items of 32 targets would be one and a half rounds of
+    blocks, and longer sums than those of 4,300; 7,000 in 64s two rounds. Each
+    must stay within 4% of the line through its neighbours (14% and 7% above it
+    otherwise)."""
+    ms = {}
+    for n in (3000, 3700, 4300, 6000, 7000, 8000):
+        s, a = spread(n, n)
+        with fss.Context(method=fss.METHOD_DIRECT) as c:
+            c.set_particles(s, a)
+            ms[n] = pair_ms(c)
+    assert ms[3700] < 1.04 * (ms[3000] + (ms[4300] - ms[3000]) * 700 / 1300), ms
+    assert ms[7000] < 1.04 * (ms[6000] + ms[8000]) / 2, ms
