@@ -240,7 +240,7 @@ int build_direct_lists(fss_ctx* c) {
         nt = std::min<int64_t>(c->fp64 ? TB : direct_group(t_end - t_first, t0 - t_first, P), t_end - t0);
         for (int p = 0; p < P; p++) {
             L.items.push_back(WorkItem{int32_t(t0), int32_t(nt), p, p + 1, p, -1,
-                                       pair_split(double(L.segs[p].b - L.segs[p].a), int(nt), c->shape.warps()),
+                                       c->fp64 ? 1 : pair_split(double(L.segs[p].b - L.segs[p].a), int(nt), c->shape.warps()),
                                        !ordered(c)});
             L.n_tiles += (L.segs[p].b - L.segs[p].a + c->shape.tile - 1) / c->shape.tile;
         }
@@ -614,6 +614,7 @@ int materialize(fss_ctx* c, PairShape shape) {
     in.parts = P;
     if (!c->fp64 && !c->member) leaf_group(c, P, in);
     c->shape.max_targets = in.group > 0 ? std::min(maxleaf, in.group + in.group / 2) : maxleaf;
+    in.fp64 = c->fp64;
     in.leaf_warps = c->shape.warps();
     in.cluster_warps = cluster_shape(c->fp64, int64_t(c->tlists.size()) * P).warps();
     in.all_leaves = c->resort;

@@ -6,6 +6,7 @@
 #include "traverse.h"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <map>
 #include <stdexcept>
@@ -323,7 +324,7 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
                 const bool last = s + 1 == subs;
                 const int32_t first = s * grp, nt = last ? nt_est - first : grp;
                 items.push_back({w * nt, WorkItem{t0 + first, last ? nt_item : grp, base, g1, p, leaf,
-                                                  pair_split(w, nt, leaf >= 0 ? in.leaf_warps : in.cluster_warps), 0}});
+                                                  in.fp64 ? 1 : pair_split(w, nt, leaf >= 0 ? in.leaf_warps : in.cluster_warps), 0}});
             }
         }
     };
@@ -382,30 +383,32 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
 // ---------------------------------------------------------------- FP32 items
 
 int pair_split(double sources, int targets, int warps) {
-    // a warp's time on a tile: 1 for 32 targets, 1.76 for 64 (two a lane), the
-    // share of the lanes that r targets left over occupy, and a fixed part
-    // for each
-    const int tile = tile_capacity(false), chunk = std::min(targets, 256);  // a pass of the kernel
-    const int full = chunk / 32, r = chunk % 32, G = full + (r > 0);
-    const double tiles = std::max(sources, 1.0) / tile;
+    // A warp's time on a tile with the targets in 1, 2 or 4 subsets, of the slowest
+    // of them: 1 for 32 targets, 1.76 for 64 (two a lane), the share of the lanes
+    // that r targets left over occupy, and a fixed part for each.
+    constexpr int kPass = 256;  // targets of a pass of the kernel
+    static const auto slowest = [] {
+        std::array<std::array<double, 3>, kPass + 1> v{};
+        for (int chunk = 0; chunk <= kPass; chunk++) {
+            const int full = chunk / 32, r = chunk % 32, G = full + (r > 0);
+            for (int k = 0, H = 1; k < 3; k++, H *= 2)
+                for (int h = 0; h < H; h++) {
+                    const int ga = G * h / H, gb = G * (h + 1) / H, f = std::min(gb, full) - ga;
+                    const double t = 1.76 * (f / 2) + (f % 2) + (gb > full ? 0.1 + 1.0 / (32 / r) : 0.0);
+                    v[chunk][k] = std::max(v[chunk][k], t);
+                }
+        }
+        return v;
+    }();
+    const double tiles = std::max(sources, 1.0) / tile_capacity(false);
     const int whole = int(tiles);
     int best = 1;
     double best_t = 1e300;
-    for (int H : {1, 2, 4}) {
-        if (warps % H) continue;
-        const int stride = warps / H;
-        double busiest = 0, slowest = 0;
-        for (int j = 0; j < stride; j++) {
-            double load = (whole - j + stride - 1) / stride;
-            if (whole % stride == j) load += tiles - whole;
-            busiest = std::max(busiest, load);
-        }
-        for (int h = 0; h < H; h++) {
-            const int ga = G * h / H, gb = G * (h + 1) / H, f = std::min(gb, full) - ga;
-            const double t = 1.76 * (f / 2) + (f % 2) + (gb > full ? 0.1 + 1.0 / (32 / r) : 0.0);
-            slowest = std::max(slowest, t);
-        }
-        const double t = busiest * (slowest + 0.1);
+    for (int k = 0, H = 1; k < 3 && warps % H == 0; k++, H *= 2) {
+        // the busiest warp's tiles: one more whole one, or the part of one
+        const int stride = warps / H, each = whole / stride;
+        const double busiest = each * stride < whole ? each + 1 : each + (tiles - whole);
+        const double t = busiest * (slowest[std::clamp(targets, 0, kPass)][k] + 0.1);
         if (t < 0.99 * best_t) {
             best_t = t;
             best = H;

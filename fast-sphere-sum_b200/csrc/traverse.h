@@ -60,8 +60,9 @@ struct ListInput {
     int tile = 256;                     // sources per shared-memory tile
     int parts = 1;                      // source-list split
     bool all_leaves = false;            // items also for leaves empty at the build
-    int leaf_warps = 4;                 // of the block that takes a leaf
-    int cluster_warps = 4;              // of the block that takes a target cluster
+    bool fp64 = false;                  // the engine that takes the items
+    int leaf_warps = 4;                 // FP32: of the block that takes a leaf
+    int cluster_warps = 4;              // FP32: of the block that takes a target cluster
     int group = 0;                      // targets per item of a leaf (a multiple of 32; 0: the whole leaf)
     bool mix = false;                   // of 16 leaves, one in items of 32 and one of 64 all the same
 };
