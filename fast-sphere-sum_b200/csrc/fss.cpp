@@ -615,6 +615,7 @@ int materialize(fss_ctx* c, PairShape shape) {
     if (!c->fp64 && !c->member) leaf_group(c, P, in);
     c->shape.max_targets = in.group > 0 ? std::min(maxleaf, in.group + in.group / 2) : maxleaf;
     in.fp64 = c->fp64;
+    in.pass = pass_targets(c->shape.max_targets);
     in.leaf_warps = c->shape.warps();
     in.cluster_warps = cluster_shape(c->fp64, int64_t(c->tlists.size()) * P).warps();
     in.all_leaves = c->resort;
@@ -1334,9 +1335,9 @@ int fss_rhs_current(fss_ctx* c, double omega, double* modify5, double* psi) {
 
 namespace {
 // Pair evaluations the lanes of a pair launch perform on items [i0, i1): every
-// 32 targets evaluate every source of the item (padded to whole quads) on
-// each lane; the last r targets split the sources over 32 / r lanes per
-// target, each lane taking every (32 / r)-th quad.
+// 32 targets of a pass evaluate every source of the item (padded to whole steps
+// of the loop) on each lane; the last r targets split the sources over 32 / r
+// lanes per target, each lane taking every (32 / r)-th step.
 double lane_pairs(const fss_ctx* c, int64_t i0, int64_t i1) {
     const ListOutput& L = c->lists;
     double sum = 0;
@@ -1347,14 +1348,19 @@ double lane_pairs(const fss_ctx* c, int64_t i0, int64_t i1) {
             const Segment& sg = L.segs[g];
             src += sg.kind == 0 ? double(c->leaf_start_h[sg.b] - c->leaf_start_h[sg.a]) : double(sg.b - sg.a);
         }
-        const double quads = std::ceil(src / 4.0);
+        const int step = c->fp64 ? 2 : 4;
+        const double steps = std::ceil(src / step);
         int nt = it.nt;
         if (it.leaf >= 0) {
             nt = std::max(0, c->leaf_start_h[it.leaf + 1] - c->leaf_start_h[it.leaf] - it.t0);
             if (it.nt > 0) nt = std::min(nt, it.nt);
         }
-        sum += 32.0 * double(nt / 32) * 4.0 * quads;
-        if (nt % 32) sum += 32.0 * 4.0 * std::ceil(quads / double(32 / (nt % 32)));
+        const int pass = c->fp64 ? chunk_targets(nt) : pass_targets(c->shape.max_targets);
+        for (int t0 = 0; t0 < nt; t0 += pass) {
+            const int cn = std::min(pass, nt - t0), r = cn % 32;
+            sum += 32.0 * step * (cn / 32) * steps;
+            if (r) sum += 32.0 * step * std::ceil(steps / double(32 / r));
+        }
     }
     return sum;
 }

@@ -412,13 +412,12 @@ __global__ void __launch_bounds__(THREADS, blocks_per_sm(THREADS))
 
 // ---------------------------------------------------------------- dispatch
 
-// Targets of one pass: leaves, target clusters and small items have at most
-// kSmallChunk; only where some have more do their totals take the larger share
-// of an SM's memory from the L1 cache, which the concurrent kernels of a step
-// use: 163,842 particles with target clusters 1,448 us per step, 1,459 with the
-// larger one; 300,001 in leaves of 234, which then take two passes, 2,838 and
-// 2,675.
-constexpr int kSmallChunk = 160, kLargeChunk = 256;
+// Targets of one pass (pass_targets): leaves, target clusters and small items
+// have at most kSmallChunk; only where some have more do their totals take the
+// larger share of an SM's memory from the L1 cache, which the concurrent kernels
+// of a step use: 163,842 particles with target clusters 1,448 us per step, 1,459
+// with the larger one; 300,001 in leaves of 234, which then take two passes,
+// 2,838 and 2,675.
 
 template <int WARPS, bool PSI, int CHUNK>
 static cudaError_t run_pairs(cudaStream_t st, int nitems, const void* src, const Segment* segs,
@@ -481,8 +480,8 @@ cudaError_t launch_pairs(cudaStream_t st, bool fp64, bool psi, PairShape shape, 
     const int warps = shape.warps();
     if (fp64)
         return launch_plane_pairs(st, psi, warps, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
-    auto run = shape.max_targets <= kSmallChunk ? (psi ? dispatch<true, kSmallChunk> : dispatch<false, kSmallChunk>)
-                                                : (psi ? dispatch<true, kLargeChunk> : dispatch<false, kLargeChunk>);
+    auto run = pass_targets(shape.max_targets) == kSmallChunk ? (psi ? dispatch<true, kSmallChunk> : dispatch<false, kSmallChunk>)
+                                                              : (psi ? dispatch<true, kLargeChunk> : dispatch<false, kLargeChunk>);
     return run(st, warps, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
 }
 

@@ -46,6 +46,10 @@ struct PairShape {
     int max_targets = 256;  // of most items (FP32: how many the block has room for)
     int warps() const { return threads / 32 - 1; }
 };
+// Targets of one pass of an FP32 block over its sources: kSmallChunk where no
+// item has more.
+constexpr int kSmallChunk = 160, kLargeChunk = 256;
+inline int pass_targets(int max_targets) { return max_targets <= kSmallChunk ? kSmallChunk : kLargeChunk; }
 
 // k_tree.cu
 void launch_assign(cudaStream_t st, int64_t n, const double* in5, const double* verts, const int32_t* tri_verts,

@@ -290,7 +290,6 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
                 if (acc >= total * p / P) cut[p++] = k + 1;
             }
         }
-        const int chunks = std::max(1, chunk_count(nt_est));
         // a leaf's targets in items of in.group, the last of them open-ended
         const int grp = !in.mix || leaf % 16 > 1 ? in.group : (leaf % 16 == 0 ? 32 : 64);
         const int subs = leaf >= 0 ? leaf_items(nt_est, grp) : 1;
@@ -317,12 +316,13 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
                     out.segs.push_back(e);
                 w += est[k];
             }
-            out.n_tiles += int64_t(std::max(chunks, subs)) * (int64_t(w + in.tile - 1) / in.tile);
             // a block's run time follows its pairs, so the most go first
             const int32_t g1 = int32_t(out.segs.size());
             for (int s = 0; s < subs; s++) {
                 const bool last = s + 1 == subs;
                 const int32_t first = s * grp, nt = last ? nt_est - first : grp;
+                const int passes = in.fp64 ? chunk_count(nt) : (nt + in.pass - 1) / in.pass;
+                out.n_tiles += passes * (int64_t(w + in.tile - 1) / in.tile);
                 items.push_back({w * nt, WorkItem{t0 + first, last ? nt_item : grp, base, g1, p, leaf,
                                                   in.fp64 ? 1 : pair_split(w, nt, leaf >= 0 ? in.leaf_warps : in.cluster_warps), 0}});
             }

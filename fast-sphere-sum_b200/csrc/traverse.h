@@ -61,6 +61,7 @@ struct ListInput {
     int parts = 1;                      // source-list split
     bool all_leaves = false;            // items also for leaves empty at the build
     bool fp64 = false;                  // the engine that takes the items
+    int pass = 256;                     // FP32: targets of one pass over an item's sources
     int leaf_warps = 4;                 // FP32: of the block that takes a leaf
     int cluster_warps = 4;              // FP32: of the block that takes a target cluster
     int group = 0;                      // targets per item of a leaf (a multiple of 32; 0: the whole leaf)

@@ -304,8 +304,10 @@ typedef struct fss_tree_info {
     double cp_interactions;  /* interpolation point-particle pairs per RHS */
     double cc_interactions;  /* interpolation point-proxy pairs per RHS */
     double lane_pairs_leaf;    /* pair evaluations the target-leaf launch's
-                                  consumer lanes perform per RHS at the build's
-                                  leaf counts, discarded lanes included */
+                                  lanes perform per RHS at the build's leaf
+                                  counts, discarded lanes included (FP64: but
+                                  for the padding of each warp's share of a
+                                  tile) */
     double lane_pairs_cluster; /* the same for the target-cluster launch */
     int32_t max_degree;        /* highest degree among the lists' proxies and
                                   target clusters (the upward pass forms

@@ -58,3 +58,33 @@ def test_moved_particles_membership(fss, oracle):
         ctx.set_particles(s, a)
         loc, _, _ = ctx.get_tree()
     assert np.array_equal(loc, loc_o)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("per_leaf", [40, 150, 165, 200, 300])
+def test_lane_pairs(fss, prec, per_leaf):
+    """The lanes' pair evaluations, from the engine's passes over the targets: FP64
+    passes of near-equal size up to 159, FP32 of 96-, 64- or 32-target items."""
+    n = 20 * per_leaf
+    rng = np.random.default_rng(per_leaf)
+    s = np.zeros((n, 5))
+    s[:, :3] = rng.standard_normal((n, 3))
+    s[:, :3] /= np.linalg.norm(s[:, :3], axis=1, keepdims=True)
+    with fss.Context(precision=prec, tree_levels=1, theta=1e-3, src_parts=1) as c:
+        c.set_particles(s, np.full(n, 4 * np.pi / n))
+        got = c.tree_info()["lane_pairs_leaf"]
+        _, counts, _ = c.get_tree()
+
+    def lanes(targets):
+        full, r = divmod(targets, 32)
+        return 32 * full + (32 / (32 // r) if r else 0)
+
+    want = 0.0
+    for nt in counts[:20]:
+        if prec == 0:
+            k = 1 if nt < 160 else -(-nt // 128)
+            size = -(-nt // k)
+        else:
+            size = 32  # items of 32: 20 to 200 of them are fewer than the blocks that run at once
+        want += sum(lanes(min(size, nt - t)) for t in range(0, nt, size)) * n
+    assert abs(got - want) < 0.01 * want + 64 * 20 * 32
