@@ -436,6 +436,7 @@ int set_particles(fss_ctx* c, int64_t n, const double* state5, const double* are
         TRY(build_direct_lists(c));
     }
     TRY(gather(c, true));
+    TRY(order_sources(c));  // a shard's combine reads the order, whether a stage came before it or not
     c->have = true;
     c->stage_dirty = false;
     if (c->tree && c->cfg.autotune) TRY(autotune(c, true));

@@ -485,7 +485,9 @@ int fss_rhs_direct_noalloc(int64_t n, const double* state5, const double* area, 
  * a target cluster, or the leaves (treecode); blocks of target rows (direct
  * sum) -- balanced by their counted interactions, so that every target
  * cluster and its downward pass lie with one rank.  Per RK stage the ranks
- * exchange one device buffer of N x 4 doubles (the context's particle order):
+ * exchange one device buffer of N x 4 doubles (the context's particle order;
+ * an FP64 direct sum of more than 15,000 particles has a spatial one that stage
+ * 1 forms from the positions, the same on every rank):
  * a rank writes the velocity sums of its own rows and -0.0 in every other
  * row; the caller sums the buffers over the ranks (an all-reduce, e.g. NCCL
  * through torch.distributed: x + -0.0 = x, so the sum is exact in any order);

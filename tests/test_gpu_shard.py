@@ -100,3 +100,40 @@ def test_one_rank_shard_equals_unsharded(fss):
         c.shard(0, 0)                         # unshard: the full lists again
         assert c.shard_info()["nranks"] == 0
     assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
+
+
+def spread(n):
+    rng = np.random.default_rng(n)
+    s = np.zeros((n, 5))
+    s[:, :3] = rng.standard_normal((n, 3))
+    s[:, :3] /= np.linalg.norm(s[:, :3], axis=1, keepdims=True)
+    s[:, 3] = rng.standard_normal(n)
+    return s, np.full(n, 4 * np.pi / n)
+
+
+def test_sharded_direct_in_spatial_order(fss):
+    """FP64 direct sums of more than 15,000 particles run in a spatial order of their own."""
+    s, a = spread(15100)
+    kw = dict(method=0, precision=0, src_parts=3)
+    with fss.Context(**kw) as c:
+        c.set_particles(s, a)
+        c.rk4_step(0.01, nsteps=2)
+        want = c.get_state()
+    states, _, _ = run_sharded(fss, kw, s, a, 2, 2)
+    assert all(np.array_equal(g, want) for g in states)
+
+
+def test_combine_without_a_stage(fss):
+    """A combine that no stage came before (zero velocities) leaves every particle
+    where it is: the spatial order it reads is that of the particles set."""
+    import torch
+    s, a = spread(15100)
+    with fss.Context(method=0, precision=0) as c:
+        c.set_particles(s, a)
+        c.shard(0, 2)
+        zero = torch.zeros((len(s), 4), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        for stage in (1, 2, 3, 4):
+            c.shard_combine(stage, 0.01, zero)
+        got = c.get_state()
+    assert np.max(np.abs(got - s)) < 1e-14
