@@ -39,15 +39,15 @@
 // pair: sources near the targets or off the sphere (kOnSphere), and every
 // source for a chunk with a target off the sphere or with targets all over it,
 // or of a direct sum in the caller's order (WorkItem::space)
-// (a tree evaluated at other positions than its own: 163,842 particles 1.33 ms,
-// where a pass over the sources around each group of targets took 4.31).
+// (a tree evaluated at other positions than its own: 163,842 particles 1.26 ms,
+// where a pass over the sources around each group of targets took 4.26).
 //
 // Bound by the FP64 pipe.  Pair sums of one right-hand side, all in space by
 // one target a lane and here: treecode of 163,842 particles (n = 8, theta =
-// 0.7) 1.320 and 0.979 ms (0.929 with all sources but the targets in the
-// plane), with target clusters (n = 10) 0.760 and 0.594; direct sum of 20,011
-// particles 0.402 and 0.323; 40,962 particles with the stream function 1.156
-// and 0.492.
+// 0.7) 1.314 and 0.960 ms (0.925 with all sources but the targets in the
+// plane), with target clusters (n = 10) 0.719 and 0.557; direct sum of 20,011
+// particles 0.402 and 0.323; 40,962 particles with the stream function 1.144
+// and 0.453.
 // The FP32 engine (k_pairs.cu) sums in space.
 #include <algorithm>
 
@@ -65,7 +65,8 @@ constexpr int kSlots = 32 * (kMaxFull + 1);  // accumulator slots of a warp
 // below which a position's rounding across the sphere would show) are near.
 // Direct sums of 2,001 to 163,842 random particles, plainly summed, come out to
 // 2.2e-16 to 5.2e-16 of the result with it as with 1.5, 2 and 3 (in space 8e-16
-// to 1.4e-14, in longer sums); the level-7 treecode above 0.979, at 1.5 0.996 ms.
+// to 1.4e-14, in longer sums); the level-7 treecode above 0.982, at 1.5 0.996 ms,
+// before the rest of its targets took a lane's next place.
 constexpr double kNear = 1.25;
 constexpr double kNearest = 1e-6;
 // What the pair loop in space adds to r^2, so that a source at the target's
@@ -280,18 +281,19 @@ __device__ __forceinline__ void space_pairs(const double4* __restrict__ s, int j
     }
 }
 
-// Such sources of a warp's share of a tile for its lanes' NT targets (tgt[32 k]),
-// added to the lane's accumulators.
+// Such sources of a warp's share of a tile for its lanes' NT targets (tgt, and
+// for NT = 2 tgt1), added to the lane's accumulators.
 template <bool PSI, int NT>
 __device__ __forceinline__ void space_fold(const double4* __restrict__ share, int j0, int n, int step,
-                                           const double4* __restrict__ tgt, Acc3* acc, double* accp,
+                                           const double4* __restrict__ tgt, const double4* __restrict__ tgt1,
+                                           Acc3* acc, double* accp,
                                            const double* lg) {
     const int lane = threadIdx.x & 31;
     double4 t[NT];
     Acc3 a[NT];
     double ap[NT];
 #pragma unroll
-    for (int k = 0; k < NT; k++) t[k] = tgt[32 * k];
+    for (int k = 0; k < NT; k++) t[k] = k == 0 ? *tgt : *tgt1;
     space_pairs<PSI, NT>(share, j0, n, step, t, a, ap, lg);
 #pragma unroll
     for (int k = 0; k < NT; k++) {
@@ -406,9 +408,9 @@ struct PairBars {
 // Warp 0 packs and issues the tiles, one ahead of the one in use.  Every warp
 // parts its share of a landed tile, sums those in space from the slot, releases
 // it through empty, and sums those in the plane, each for all targets of the
-// chunk: cn >> 5 targets a
-// lane (a source loaded serves them all) and, for the r = cn & 31 left over,
-// L = 32 / r lanes a target, which split the share between them.  So the
+// chunk: cn >> 5 targets a lane (a source loaded serves them all) and, for the
+// r = cn & 31 left over, L = 32 / r lanes a target, which split the share
+// between them, or one more target a lane where L is 1 anyway.  So the
 // warps' work is equal whatever the count of targets (one warp per 32 targets
 // left the SM's quarters unequally loaded: leaves of 78 particles ran at 62%
 // of the rate of leaves of 128), and no warp waits for another's mapping.
@@ -431,7 +433,8 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
     const int chunk = chunk_targets(nt);
     for (int c0 = 0; c0 < nt; c0 += chunk) {
         const int cn = min(chunk, nt - c0);
-        const int full = cn >> 5, r = cn & 31;
+        const int merge = (cn & 31) > 16 && (cn >> 5) < kMaxFull ? 1 : 0;  // the rest as one more a lane
+        const int full = (cn >> 5) + merge, r = merge ? 0 : cn & 31;
         const int L = r > 0 ? 32 / r : 1;
         // warp 0: the next tile into its slot (an empty one ends the chunk),
         // once every warp has mapped the tile before it there
@@ -500,8 +503,8 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
         if (!it.space) {
             Plane plane;
             plane.load(*ps);
-            for (int i = tid; i < cn; i += 32 * WARPS) {
-                const double4 v = src[t0 + c0 + i];
+            for (int i = tid; i < max(cn, 32 * full); i += 32 * WARPS) {
+                const double4 v = src[t0 + c0 + min(i, cn - 1)];
                 double2 p;
                 plane_map(plane, v.x, v.y, v.z, p.x, p.y);
                 sm.tpos[i] = p;
@@ -544,13 +547,13 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const double4* __re
                 const double4* tgt = src + t0 + c0;
                 int g = 0;
                 for (; g + 2 <= full; g += 2)
-                    space_fold<PSI, 2>(share, 0, nn, 1, tgt + 32 * g + lane, acc3 + 32 * g,
-                                       PSI ? accp + 32 * g : accp, sm.lg);
+                    space_fold<PSI, 2>(share, 0, nn, 1, tgt + 32 * g + lane, tgt + min(32 * g + 32 + lane, cn - 1),
+                                       acc3 + 32 * g, PSI ? accp + 32 * g : accp, sm.lg);
                 if (g < full)
-                    space_fold<PSI, 1>(share, 0, nn, 1, tgt + 32 * g + lane, acc3 + 32 * g,
+                    space_fold<PSI, 1>(share, 0, nn, 1, tgt + min(32 * g + lane, cn - 1), nullptr, acc3 + 32 * g,
                                        PSI ? accp + 32 * g : accp, sm.lg);
                 if (r > 0)
-                    space_fold<PSI, 1>(share, lane % L, nn, L, tgt + 32 * full + min(lane / L, r - 1),
+                    space_fold<PSI, 1>(share, lane % L, nn, L, tgt + 32 * full + min(lane / L, r - 1), nullptr,
                                        acc3 + 32 * full, PSI ? accp + 32 * full : accp, sm.lg);
             }
             __syncwarp();
