@@ -79,7 +79,6 @@ struct fss_ctx {
     ListOutput lists;
     std::vector<std::vector<ASrc>> alists;  // per-leaf sources before packing
     std::vector<fss::TList> tlists;         // target clusters (cp/cc) and their sources
-    std::vector<std::pair<fss::PairShape, double>> tuned;  // autotuner: shape, ms per pair pass
     std::vector<std::pair<int, double>> tuned_depth;       // autotuner: tree levels, ms per RHS
     std::vector<std::pair<int, double>> tuned_parts;       // autotuner: src_parts, ms per right-hand side
     int64_t depth_n = -1;  // particle count the tuned depth belongs to

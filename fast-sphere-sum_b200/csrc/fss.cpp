@@ -206,7 +206,7 @@ bool ordered(const fss_ctx* c) { return !c->tree && c->fp64 && c->n > kOrderFrom
 // Lists of the direct sum: blocks of targets x P chunks of the sources.
 int build_direct_lists(fss_ctx* c) {
     const int64_t n = c->n;
-    c->shape = pairs_shape(c->fp64, c->cfg.block_threads, c->cfg.targets_per_thread);
+    c->shape = pairs_shape(c->fp64, c->cfg.block_threads);
     const int TB = c->fp64 ? kChunkTargets : c->shape.threads - 32;
     const int64_t tiles = (n + TB - 1) / TB;
     int P = c->cfg.src_parts;
@@ -240,7 +240,7 @@ int build_direct_lists(fss_ctx* c) {
         nt = std::min<int64_t>(c->fp64 ? TB : direct_group(t_end - t_first, t0 - t_first, P), t_end - t0);
         for (int p = 0; p < P; p++) {
             L.items.push_back(WorkItem{int32_t(t0), int32_t(nt), p, p + 1, p, -1,
-                                       c->fp64 ? 1 : pair_split(double(L.segs[p].b - L.segs[p].a), int(nt), c->shape.warps()),
+                                       c->fp64 ? 1 : pair_split(double(L.segs[p].b - L.segs[p].a), int(nt), c->shape.warps),
                                        !ordered(c)});
             L.n_tiles += (L.segs[p].b - L.segs[p].a + c->shape.tile - 1) / c->shape.tile;
         }
@@ -439,7 +439,7 @@ int set_particles(fss_ctx* c, int64_t n, const double* state5, const double* are
     TRY(order_sources(c));  // a shard's combine reads the order, whether a stage came before it or not
     c->have = true;
     c->stage_dirty = false;
-    if (c->tree && c->cfg.autotune) TRY(autotune(c, true));
+    if (c->tree && c->cfg.autotune >= 2) TRY(autotune(c, true));
     TRY(refresh_stage(c));
     return check_device_error(c);
 }
@@ -547,7 +547,7 @@ int build_tree(fss_ctx* c) {
 // Block shape for the treecode's pair kernel: the configured one, or the
 // smallest.
 PairShape choose_shape(fss_ctx* c) {
-    return pairs_shape(c->fp64, c->cfg.block_threads, c->cfg.targets_per_thread);
+    return pairs_shape(c->fp64, c->cfg.block_threads);
 }
 
 // FP32 engine: targets per item of a leaf whose lists are split into `parts`.
@@ -617,8 +617,8 @@ int materialize(fss_ctx* c, PairShape shape) {
     c->shape.max_targets = in.group > 0 ? std::min(maxleaf, in.group + in.group / 2) : maxleaf;
     in.fp64 = c->fp64;
     in.pass = pass_targets(c->shape.max_targets);
-    in.leaf_warps = c->shape.warps();
-    in.cluster_warps = cluster_shape(c->fp64, int64_t(c->tlists.size()) * P).warps();
+    in.leaf_warps = c->shape.warps;
+    in.cluster_warps = cluster_shape(c->fp64, int64_t(c->tlists.size()) * P).warps;
     in.all_leaves = c->resort;
     c->parts = P;
     build_lists(in, c->alists, c->tlists, c->lists);
@@ -893,26 +893,23 @@ int tune_rhs(fss_ctx* c) {
     return eval(c, ea, false);
 }
 
-// Autotuner, run by fss_set_particles.  autotune >= 1: the pair kernel's
-// block shape -- every supported shape timed on the current lists (after
-// the upward pass), the fastest kept.  autotune >= 2 also: the tree depth
-// (leaf size), when the configuration leaves it automatic -- the automatic
-// depth and one level either side, each built and timed on a whole
-// right-hand side (the fastest is kept for this particle count); and the
-// source split (src_parts 1, 2, 4 and, in FP64, whose automatic split goes
-// further, that one and its neighbours), when automatic, timed on a whole
-// right-hand side (more parts balance the pair launches but add partial slots
-// for the epilogue to sum).
+// Autotuner, run by fss_set_particles with autotune >= 2 (1 has nothing to
+// choose: every pair launch has its one block shape): the tree depth (leaf size),
+// when the configuration leaves it automatic -- the automatic depth and one
+// level either side, each built and timed on a whole right-hand side (the fastest
+// is kept for this particle count); and the source split (src_parts 1, 2, 4 and,
+// in FP64, whose automatic split goes further, that one and its neighbours), when
+// automatic, timed on a whole right-hand side (more parts balance the pair
+// launches but add partial slots for the epilogue to sum).
 // depth = false (lists rebuilt for per-leaf parameters, which belong to the
 // current leaves) keeps the tree.
 int autotune(fss_ctx* c, bool depth) {
-    c->tuned.clear();
     const bool prof_was = c->prof;
     c->prof = false;
     TuneEvents ev;
     CU(cudaEventCreate(&ev.a));
     CU(cudaEventCreate(&ev.b));
-    if (depth && c->cfg.autotune >= 2 && c->tree && c->cfg.tree_levels == 0 && c->depth_n != c->n) {
+    if (depth && c->cfg.tree_levels == 0 && c->depth_n != c->n) {
         const int base = c->tree_levels;
         int best_tl = base;
         double best_ms = 1e30;
@@ -939,21 +936,7 @@ int autotune(fss_ctx* c, bool depth) {
             c->stage_dirty = false;
         }
     }
-    PairShape best = c->shape;
-    double best_ms = 1e30;
-    for (const PairShape& sh : pair_shapes(c->fp64)) {
-        TRY(materialize(c, sh));
-        TRY(refresh_stage(c));
-        TRY(tune_rhs(c));  // proxies of the upward pass for the pair launches
-        double ms = 0;
-        TRY(time_ms(c, ev, 2, [&] { return launch_all_pairs(c, false); }, &ms));
-        c->tuned.push_back({sh, ms});
-        if (ms < best_ms) {
-            best_ms = ms;
-            best = sh;
-        }
-    }
-    if (c->cfg.autotune >= 2 && c->cfg.src_parts == 0) {
+    if (c->cfg.src_parts == 0) {
         c->tuned_parts.clear();
         int best_p = 1;
         double best_p_ms = 1e30;
@@ -963,7 +946,7 @@ int autotune(fss_ctx* c, bool depth) {
                 if (p >= 1 && std::find(splits.begin(), splits.end(), p) == splits.end()) splits.push_back(p);
         for (int p : splits) {
             c->cfg.src_parts = p;
-            TRY(materialize(c, best));
+            TRY(materialize(c, c->shape));
             TRY(refresh_stage(c));
             double ms = 0;
             TRY(time_ms(c, ev, 3, [&] { return tune_rhs(c); }, &ms));
@@ -975,7 +958,7 @@ int autotune(fss_ctx* c, bool depth) {
         }
         c->cfg.src_parts = best_p;
     }
-    TRY(materialize(c, best));
+    TRY(materialize(c, c->shape));
     c->prof = prof_was;
     c->stage_dirty = true;  // the timing passes overwrote the stage sources
     return FSS_OK;
@@ -1116,12 +1099,10 @@ int internal_relist(fss_ctx* c) {
     invalidate_graph(c);
     make_alists(c, c->counts_h);
     TRY(shard_filter(c));
+    if (c->cfg.autotune >= 2 && c->src_parts_given == 0) c->cfg.src_parts = 0;  // tuned again for the new lists
     TRY(materialize(c, choose_shape(c)));
     c->stage_dirty = true;
-    if (c->cfg.autotune) {  // block shape (and source split) for the new lists
-        if (c->cfg.autotune >= 2 && c->src_parts_given == 0) c->cfg.src_parts = 0;  // tune it again
-        TRY(autotune(c, false));
-    }
+    if (c->cfg.autotune >= 2) TRY(autotune(c, false));
     TRY(refresh_stage(c));
     return check_device_error(c);
 }
@@ -1382,7 +1363,7 @@ int fss_get_tree_info(fss_ctx* c, fss_tree_info* info) {
     info->pp_interactions = c->lists.pp_pairs;
     info->pc_interactions = c->lists.pc_pairs;
     info->block_threads = c->shape.threads;
-    info->targets_per_thread = c->shape.per_thread;
+    info->targets_per_thread = 1;
     info->src_parts = c->parts;
     info->target_clusters = int32_t(c->lists.down.size());
     info->cp_interactions = c->lists.cp_pairs;

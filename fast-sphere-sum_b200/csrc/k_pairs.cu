@@ -431,21 +431,11 @@ static cudaError_t run_pairs(cudaStream_t st, int nitems, const void* src, const
     return cudaGetLastError();
 }
 
-const std::vector<PairShape>& pair_shapes(bool fp64) {
-    static const auto shapes = [](int tile) {
-        std::vector<PairShape> v;
-        for (int threads : {160, 192, 224, 288}) v.push_back({threads, 1, tile, 256});
-        return v;
-    };
-    static const std::vector<PairShape> f32 = shapes(tile_capacity(false)), f64 = shapes(tile_capacity(true));
-    return fp64 ? f64 : f32;
-}
-
-PairShape pairs_shape(bool fp64, int threads, int per_thread) {
-    (void)per_thread;
-    for (const PairShape& s : pair_shapes(fp64))
-        if (s.threads == threads) return s;
-    return pair_shapes(fp64).front();
+PairShape pairs_shape(bool fp64, int threads) {
+    PairShape s;
+    s.tile = tile_capacity(fp64);
+    if (threads == 192 || threads == 224 || threads == 288) s.threads = threads;
+    return s;
 }
 
 // FP32: four warps when all items run at once anyway (740 such blocks fit; us
@@ -453,8 +443,8 @@ PairShape pairs_shape(bool fp64, int threads, int per_thread) {
 // smaller pieces of work beside the leaves' launch (420 in 4 parts 394, with four
 // warps 416; 6,820 4,032 and 4,126).
 PairShape cluster_shape(bool fp64, int64_t items) {
-    PairShape s = pair_shapes(fp64).front();
-    if (!fp64 && items >= 740) s.threads = 96;
+    PairShape s = pairs_shape(fp64, 0);
+    if (!fp64 && items >= 740) s.warps = 2;
     s.max_targets = kMaxK;
     return s;
 }
@@ -463,13 +453,7 @@ template <bool PSI, int CHUNK>
 static cudaError_t dispatch(cudaStream_t st, int warps, int nitems, const void* src, const Segment* segs,
                             const int32_t* leaf_start, const WorkItem* items, double4* partials, int64_t pstride,
                             int* err, PairCtl ctl) {
-    auto run = warps == 2   ? run_pairs<2, PSI, CHUNK>
-               : warps == 4 ? run_pairs<4, PSI, CHUNK>
-               : warps == 5 ? run_pairs<5, PSI, CHUNK>
-               : warps == 6 ? run_pairs<6, PSI, CHUNK>
-               : warps == 8 ? run_pairs<8, PSI, CHUNK>
-                            : nullptr;
-    if (!run) return cudaErrorInvalidConfiguration;
+    auto run = warps == 2 ? run_pairs<2, PSI, CHUNK> : run_pairs<4, PSI, CHUNK>;
     return run(st, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
 }
 
@@ -477,12 +461,11 @@ cudaError_t launch_pairs(cudaStream_t st, bool fp64, bool psi, PairShape shape, 
                          const Segment* segs, const int32_t* leaf_start, const WorkItem* items,
                          double4* partials, int64_t pstride, int* err, PairCtl ctl) {
     if (nitems == 0) return cudaSuccess;
-    const int warps = shape.warps();
     if (fp64)
-        return launch_plane_pairs(st, psi, warps, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
+        return launch_plane_pairs(st, psi, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
     auto run = pass_targets(shape.max_targets) == kSmallChunk ? (psi ? dispatch<true, kSmallChunk> : dispatch<false, kSmallChunk>)
                                                               : (psi ? dispatch<true, kLargeChunk> : dispatch<false, kLargeChunk>);
-    return run(st, warps, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
+    return run(st, shape.warps, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
 }
 
 cudaError_t launch_pairs_persistent(cudaStream_t st, int nitems, const void* src, const Segment* segs,

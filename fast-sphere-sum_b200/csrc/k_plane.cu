@@ -691,25 +691,12 @@ static cudaError_t run_pairs(cudaStream_t st, int nitems, const void* src, const
     return cudaGetLastError();
 }
 
-template <bool PSI>
-static cudaError_t dispatch(cudaStream_t st, int warps, int nitems, const void* src, const Segment* segs,
-                            const int32_t* leaf_start, const WorkItem* items, double4* partials, int64_t pstride,
-                            int* err, PairCtl ctl) {
-    switch (warps) {
-        case 4: return run_pairs<128, PSI>(st, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
-        case 5: return run_pairs<160, PSI>(st, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
-        case 6: return run_pairs<192, PSI>(st, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
-        case 8: return run_pairs<256, PSI>(st, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
-    }
-    return cudaErrorInvalidConfiguration;
-}
-
-cudaError_t launch_plane_pairs(cudaStream_t st, bool psi, int warps, int nitems, const void* src, const Segment* segs,
+cudaError_t launch_plane_pairs(cudaStream_t st, bool psi, int nitems, const void* src, const Segment* segs,
                                const int32_t* leaf_start, const WorkItem* items, double4* partials, int64_t pstride,
                                int* err, PairCtl ctl) {
     if (nitems == 0) return cudaSuccess;
-    return psi ? dispatch<true>(st, warps, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl)
-               : dispatch<false>(st, warps, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
+    auto run = psi ? run_pairs<128, true> : run_pairs<128, false>;
+    return run(st, nitems, src, segs, leaf_start, items, partials, pstride, err, ctl);
 }
 
 }  // namespace fss

@@ -38,13 +38,12 @@ struct EpiArgs {
     const int32_t* order = nullptr;
 };
 
-// Pair-kernel block: threads / 32 - 1 warps, which share an item's sources.
+// A pair launch: blocks of `warps` warps, which share an item's sources.
 struct PairShape {
-    int threads = 160;
-    int per_thread = 1;
+    int warps = 4;
+    int threads = 160;  // the configuration's block_threads: blocks of threads - 32 targets in the source split
     int tile = 256;
     int max_targets = 256;  // of most items (FP32: how many the block has room for)
-    int warps() const { return threads / 32 - 1; }
 };
 // Targets of one pass of an FP32 block over its sources: kSmallChunk where no
 // item has more.
@@ -92,17 +91,18 @@ void launch_gather(cudaStream_t st, bool fp64, int64_t n, const double* in5, con
                    double* tracer_s, void* src);
 
 // k_pairs.cu
-// Block shapes of the pair kernel the autotuner tries.
-const std::vector<PairShape>& pair_shapes(bool fp64);
-// The supported shape with `threads`, or the default (160).
-PairShape pairs_shape(bool fp64, int threads, int per_thread);
+// The shape for block_threads (160, 192, 224 or 288; else 160).  Four warps
+// whatever it is: five, six or eight (with as many registers) are 0 to 16%
+// slower, since 2 and 4 subsets of an item's targets do not divide them or an SM
+// holds fewer.
+PairShape pairs_shape(bool fp64, int threads);
 // Block for `items` target clusters (times source parts).
 PairShape cluster_shape(bool fp64, int64_t items);
 cudaError_t launch_pairs(cudaStream_t st, bool fp64, bool psi, PairShape shape, int nitems, const void* src,
                          const Segment* segs, const int32_t* leaf_start, const WorkItem* items, double4* partials,
                          int64_t pstride, int* err, PairCtl ctl);
 // The FP64 engine (k_plane.cu), launched by launch_pairs.
-cudaError_t launch_plane_pairs(cudaStream_t st, bool psi, int warps, int nitems, const void* src, const Segment* segs,
+cudaError_t launch_plane_pairs(cudaStream_t st, bool psi, int nitems, const void* src, const Segment* segs,
                                const int32_t* leaf_start, const WorkItem* items, double4* partials, int64_t pstride,
                                int* err, PairCtl ctl);
 constexpr int kPersistentThreads = 128;

@@ -99,19 +99,20 @@ typedef struct fss_config {
     int32_t use_graph;     /* capture the RK4 step in a CUDA graph */
     int32_t src_parts;     /* split each target's source list in this many parts
                               (0 = automatic) */
-    int32_t block_threads; /* shape of an interaction block: 160, 192, 224 or
-                              288 for 4, 5, 6 or 8 warps (0 = automatic: 4) */
+    int32_t block_threads; /* 160, 192, 224 or 288: blocks of 32 targets fewer in
+                              the automatic source split and in a sharded direct
+                              sum (0 = automatic).  The kernels' blocks have
+                              their own sizes. */
     int32_t targets_per_thread; /* 1 */
-    int32_t autotune;      /* at fss_set_particles: 1 = time every supported
-                              block shape of the pair kernel on the actual
-                              lists and keep the fastest; 2 = also, when
+    int32_t autotune;      /* at fss_set_particles: 2 = choose by timing, when
                               tree_levels is 0, the tree depth (leaf size: the
                               automatic depth and one level either side, each
                               timed on a whole right-hand side, the fastest kept
                               for this particle count) and, when src_parts is
                               0, the source split (1, 2, 4 and, in FP64, the
                               automatic split and the two next to it: the
-                              fastest kept) */
+                              fastest kept); 1 = nothing is left to choose (it
+                              timed the pair kernel's block shapes) */
     int32_t rebuild;       /* fss_rebuild_policy */
     int32_t cluster_targets; /* 1 = the reference's cp/cc interaction types
                               (fast_rhs.h cp, cc): a well-separated target face
@@ -297,7 +298,7 @@ typedef struct fss_tree_info {
     int64_t unassigned;      /* particles without a leaf (reference mode) */
     double pp_interactions;  /* particle-particle pair count per RHS */
     double pc_interactions;  /* particle-proxy pair count per RHS */
-    int32_t block_threads;   /* pair-kernel block shape in use */
+    int32_t block_threads;   /* the configuration's (0: 160) */
     int32_t targets_per_thread;
     int32_t src_parts;
     int32_t target_clusters; /* faces evaluated at interpolation points (cp/cc) */

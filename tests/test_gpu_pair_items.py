@@ -121,3 +121,17 @@ def test_direct_items_fit_one_round(fss):
             ms[n] = pair_ms(c)
     assert ms[3700] < 1.04 * (ms[3000] + (ms[4300] - ms[3000]) * 700 / 1300), ms
     assert ms[7000] < 1.04 * (ms[6000] + ms[8000]) / 2, ms
+
+
+@pytest.mark.parametrize("block", [160, 192, 224, 288])
+@pytest.mark.parametrize("clusters", [0, 1])
+def test_block_threads_cost_nothing(fss, block, clusters):
+    """block_threads counts in the source split only: with the split given, the
+    sums take the same time (five, six and eight warps took up to 16% longer)."""
+    s, a = spread(40962, 5)
+    ms = []
+    for b in (0, block):
+        with fss.Context(block_threads=b, src_parts=4, cluster_targets=clusters) as c:
+            c.set_particles(s, a)
+            ms.append(pair_ms(c))
+    assert ms[1] < 1.04 * ms[0]
