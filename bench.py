@@ -215,8 +215,8 @@ def time_steps(ctx, stream, steps, flush):
 
 
 def make_arm(fss, state, area, stream, prec, args, dev, clusters=False):
-    """Fixed degree/theta treecode; tree depth, source split and block shape
-    chosen by the autotuner."""
+    """Fixed degree/theta treecode; tree depth and source split chosen by the
+    autotuner."""
     ctx = fss.Context(method=fss.METHOD_TREECODE, precision=prec, degree=args.degree, theta=args.theta,
                       cluster_targets=int(clusters), device=dev, autotune=2)
     ctx.set_stream(stream.cuda_stream)
@@ -236,10 +236,9 @@ def auto_tree_levels(n, leaf_target=64, max_levels=8):
 
 def make_learned_arm(fss, state, area, stream, args, dev, clusters=True):
     """Mixed precision with the learned per-leaf (degree, theta) (with target
-    clusters: carried up to the faces of a dual traversal); block shape and
-    source split chosen by the autotuner on the learned lists (the tree
-    depth stays the automatic one, on which the selector's network was
-    trained)."""
+    clusters: carried up to the faces of a dual traversal); source split
+    chosen by the autotuner on the learned lists (the tree depth stays the
+    automatic one, on which the selector's network was trained)."""
     from fss_b200 import selector
     ctx = fss.Context(method=fss.METHOD_TREECODE, precision=fss.PREC_MIXED, list_mode=fss.LIST_LEAF,
                       cluster_targets=int(clusters), degree=args.degree, theta=args.theta, device=dev, autotune=2,
