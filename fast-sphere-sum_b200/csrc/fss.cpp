@@ -153,10 +153,10 @@ int src_size_ensure(fss_ctx* c, int64_t count) {
 // go through `sources` sources each, that takes the least time where an SM
 // shares its FP64 pipe between its blocks and up to three run side by side
 // unhindered, and a block's start and final sum cost as much as 100 sources.
-// Measured against every split of 1 to 16 (us per right-hand side, FP64
-// treecode): 20 leaves of 128 16 parts 62.1 (4 parts 65.1), 80 leaves of 250
-// 12 parts 167.9 (4: 205.3), 320 of 128 5 parts 242 (4: 243.7), 1280 of 128 3
-// parts 981 (2: 1003.5); never more than 2% behind the best one.
+// Measured against splits of 1 to 16 (us per right-hand side, FP64 treecode):
+// 20 leaves of 128 16 parts 55.1 (4 parts 60.9), 80 leaves of 250 12 parts 169.0
+// (11, its choice, 173.3; 4: 206.3), 320 of 128 5 parts 243.5 (4: 247.8), 1280 of
+// 128 3 parts 1025 (2: 1041); never more than 4% behind the best one.
 int plane_parts(double blocks, double sources, int most) {
     int best = 1;
     double best_t = 1e300;
