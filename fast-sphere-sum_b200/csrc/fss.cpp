@@ -206,7 +206,7 @@ bool ordered(const fss_ctx* c) { return !c->tree && c->fp64 && c->n > kOrderFrom
 // Lists of the direct sum: blocks of targets x P chunks of the sources.
 int build_direct_lists(fss_ctx* c) {
     const int64_t n = c->n;
-    c->shape = pairs_shape(c->fp64, c->cfg.block_threads);
+    c->shape = pairs_shape(c->cfg.block_threads);
     const int TB = c->fp64 ? kChunkTargets : c->shape.threads - 32;
     const int64_t tiles = (n + TB - 1) / TB;
     int P = c->cfg.src_parts;
@@ -242,7 +242,7 @@ int build_direct_lists(fss_ctx* c) {
             L.items.push_back(WorkItem{int32_t(t0), int32_t(nt), p, p + 1, p, -1,
                                        c->fp64 ? 1 : pair_split(double(L.segs[p].b - L.segs[p].a), int(nt), c->shape.warps),
                                        !ordered(c)});
-            L.n_tiles += (L.segs[p].b - L.segs[p].a + c->shape.tile - 1) / c->shape.tile;
+            L.n_tiles += (L.segs[p].b - L.segs[p].a + kTileSources - 1) / kTileSources;
         }
     }
     L.n_leaf_items = int64_t(L.items.size());
@@ -547,7 +547,7 @@ int build_tree(fss_ctx* c) {
 // Block shape for the treecode's pair kernel: the configured one, or the
 // smallest.
 PairShape choose_shape(fss_ctx* c) {
-    return pairs_shape(c->fp64, c->cfg.block_threads);
+    return pairs_shape(c->cfg.block_threads);
 }
 
 // FP32 engine: targets per item of a leaf whose lists are split into `parts`.
@@ -560,8 +560,10 @@ PairShape choose_shape(fss_ctx* c) {
 // 80 of 128 37.3 36.7 31.6 31.1; 80 of 250 109 72.3 72.2 73.1; 320 of 218 251
 // 230 233 249; 1280 of 128 527 517 541 565; 5120 of 128 2473 2438 2533 2693;
 // 20 of 32 11.4 (whole) 12.5 (32).  With 1 to 4 rounds of blocks, some leaves
-// in 64s and 32s leave a finer tail (items start in the order of their pairs):
-// 1332 -> 1291 us per step of 100,003 particles.  Where target clusters'
+// in 64s and 32s leave a finer tail (items start in the order of their pairs); us
+// per step without and with them: 29,634 particles 408 397, 34,672 464 435, 47,463
+// 612 610, 64,972 903 887, 88,941 1138 1107, 100,003 1332 1291, 142,449 1926 1842
+// (the last within four rounds).  Where target clusters'
 // launches fill the SMs as well, leaves of less than 192 stay whole and larger
 // ones are cut in 128s: per step 40,962 particles in leaves of 128 394 us (in 96s
 // and 128s 410); 20,011 in leaves of 250 286 us (whole 352).
@@ -597,7 +599,6 @@ int materialize(fss_ctx* c, PairShape shape) {
     in.leaf_level = LL;
     in.n = n;
     in.leaf_start = c->leaf_start_h.data();
-    in.tile = shape.tile;
     int P = c->cfg.src_parts, maxleaf = 1;
     for (int64_t l = 0; l < c->nleaf; l++) maxleaf = std::max(maxleaf, c->leaf_start_h[l + 1] - c->leaf_start_h[l]);
     if (P <= 0) {

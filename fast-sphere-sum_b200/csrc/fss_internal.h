@@ -70,11 +70,8 @@ struct PairCtl {
     int32_t pad;
 };
 
-// Sources per shared-memory tile: 256 float4 (4 KB) or 256 double4 (8 KB).
-FSS_HD constexpr int tile_capacity(bool fp64) {
-    (void)fp64;
-    return 256;
-}
+// Sources per shared-memory tile (float4: 4 KB, double4: 8 KB).
+constexpr int kTileSources = 256;
 
 // Upward-pass combine work: node `node` (global index, levels concatenated)
 // on `level`; proxies of degree set `degmask` (bit d = degree d) written at

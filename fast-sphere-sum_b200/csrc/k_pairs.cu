@@ -46,7 +46,7 @@ namespace fss {
 // (eight: the sums of 163,842 particles 832 us instead of 690, with target
 // clusters 434 instead of 330).
 constexpr int unroll(bool psi, int targets) { return psi ? 2 : (targets == 1 ? 4 : 8); }
-constexpr int kTile = tile_capacity(false);
+constexpr int kTile = kTileSources;
 constexpr float kSelfR2 = 1e-30f;  // r^2 bias of the pair loop (a normal float; 1 / kSelfR2 finite)
 
 // Sums of a tile in structure-of-arrays order (x[kTile], y, z, w, padded to a
@@ -431,9 +431,8 @@ static cudaError_t run_pairs(cudaStream_t st, int nitems, const void* src, const
     return cudaGetLastError();
 }
 
-PairShape pairs_shape(bool fp64, int threads) {
+PairShape pairs_shape(int threads) {
     PairShape s;
-    s.tile = tile_capacity(fp64);
     if (threads == 192 || threads == 224 || threads == 288) s.threads = threads;
     return s;
 }
@@ -443,7 +442,7 @@ PairShape pairs_shape(bool fp64, int threads) {
 // smaller pieces of work beside the leaves' launch (420 in 4 parts 394, with four
 // warps 416; 6,820 4,032 and 4,126).
 PairShape cluster_shape(bool fp64, int64_t items) {
-    PairShape s = pairs_shape(fp64, 0);
+    PairShape s;
     if (!fp64 && items >= 740) s.warps = 2;
     s.max_targets = kMaxK;
     return s;

@@ -42,7 +42,6 @@ struct EpiArgs {
 struct PairShape {
     int warps = 4;
     int threads = 160;  // the configuration's block_threads: blocks of threads - 32 targets in the source split
-    int tile = 256;
     int max_targets = 256;  // of most items (FP32: how many the block has room for)
 };
 // Targets of one pass of an FP32 block over its sources: kSmallChunk where no
@@ -95,7 +94,7 @@ void launch_gather(cudaStream_t st, bool fp64, int64_t n, const double* in5, con
 // whatever it is: five, six or eight (with as many registers) are 0 to 16%
 // slower, since 2 and 4 subsets of an item's targets do not divide them or an SM
 // holds fewer.
-PairShape pairs_shape(bool fp64, int threads);
+PairShape pairs_shape(int threads);
 // Block for `items` target clusters (times source parts).
 PairShape cluster_shape(bool fp64, int64_t items);
 cudaError_t launch_pairs(cudaStream_t st, bool fp64, bool psi, PairShape shape, int nitems, const void* src,

@@ -322,7 +322,7 @@ void build_lists(const ListInput& in, const std::vector<std::vector<ASrc>>& list
                 const bool last = s + 1 == subs;
                 const int32_t first = s * grp, nt = last ? nt_est - first : grp;
                 const int passes = in.fp64 ? chunk_count(nt) : (nt + in.pass - 1) / in.pass;
-                out.n_tiles += passes * (int64_t(w + in.tile - 1) / in.tile);
+                out.n_tiles += passes * (int64_t(w + kTileSources - 1) / kTileSources);
                 items.push_back({w * nt, WorkItem{t0 + first, last ? nt_item : grp, base, g1, p, leaf,
                                                   in.fp64 ? 1 : pair_split(w, nt, leaf >= 0 ? in.leaf_warps : in.cluster_warps), 0}});
             }
@@ -400,7 +400,7 @@ int pair_split(double sources, int targets, int warps) {
         }
         return v;
     }();
-    const double tiles = std::max(sources, 1.0) / tile_capacity(false);
+    const double tiles = std::max(sources, 1.0) / kTileSources;
     const int whole = int(tiles);
     int best = 1;
     double best_t = 1e300;

@@ -57,7 +57,6 @@ struct ListInput {
     int leaf_level = 0;                 // tree_levels - 1
     int64_t n = 0;                      // particles
     const int32_t* leaf_start = nullptr;  // nleaf + 1 (sorted order) at the build; estimates only
-    int tile = 256;                     // sources per shared-memory tile
     int parts = 1;                      // source-list split
     bool all_leaves = false;            // items also for leaves empty at the build
     bool fp64 = false;                  // the engine that takes the items
