@@ -37,17 +37,17 @@
 // the map holds on the unit sphere alone and serves targets on c's side of it
 // (kMinCos).  What it does not serve is summed in space, at 14 operations a
 // pair: sources near the targets or off the sphere (kOnSphere), and every
-// source for a chunk with a target off the sphere or with targets all over it,
-// or of a direct sum in the caller's order (WorkItem::space)
-// (a tree evaluated at other positions than its own: 163,842 particles 1.26 ms,
-// where a pass over the sources around each group of targets took 4.26).
+// source of a direct sum in the caller's order (WorkItem::space) or for a chunk
+// with a target off the sphere or with targets all over it (a tree evaluated at
+// other positions than its own: 163,842 particles 1.26 ms, where a pass over the
+// sources around each group of targets took 4.26).
 //
-// Bound by the FP64 pipe.  Pair sums of one right-hand side, all in space by
-// one target a lane and here: treecode of 163,842 particles (n = 8, theta =
-// 0.7) 1.314 and 0.960 ms (0.925 with all sources but the targets in the
-// plane), with target clusters (n = 10) 0.719 and 0.557; direct sum of 20,011
-// particles 0.402 and 0.323; 40,962 particles with the stream function 1.144
-// and 0.453.
+// Bound by the FP64 pipe, 79% busy in the first of these.  Pair sums of one
+// right-hand side, all in space by one target a lane and here: treecode of
+// 163,842 particles (n = 8, theta = 0.7) 1.314 and 0.960 ms (0.925 with all
+// sources but the targets in the plane), with target clusters (n = 10) 0.719 and
+// 0.557; direct sum of 20,011 particles 0.402 and 0.323; 40,962 particles with the
+// stream function 1.144 and 0.453.
 // The FP32 engine (k_pairs.cu) sums in space.
 #include <algorithm>
 
